@@ -366,30 +366,6 @@ __global__ void __launch_bounds__(256) k_unfold(const T* __restrict__ spec, int 
     }
 }
 
-// alm[b][l][m] (complex) -> almT[m][l][c], c = 2b + {re, im}
-template <typename T>
-__global__ void k_alm_to_cols(const T* __restrict__ alm, int nmaps, int L, int M, T* __restrict__ almT, int C) {
-    __shared__ cplx<T> tile[16][33];
-    const int m0 = blockIdx.x * 32, l = blockIdx.y, b0 = blockIdx.z * 16;
-    const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-    for (int i = ty; i < 16; i += 8) {
-        const int b = b0 + i, m = m0 + tx;
-        cplx<T> v = {(T)0, (T)0};
-        if (b < nmaps && m < M) v = *(const cplx<T>*)(alm + 2 * (((int64_t)b * L + l) * M + m));
-        tile[i][tx] = v;
-    }
-    __syncthreads();
-    // write: for each m in tile, 32 consecutive columns (16 maps x re/im)
-    for (int i = ty; i < 32; i += 8) {
-        const int m = m0 + i;
-        const int c = 2 * b0 + tx;
-        if (m < M && c < C) {
-            cplx<T> v = tile[tx >> 1][i];
-            almT[((int64_t)m * L + l) * C + c] = (tx & 1) ? v.im : v.re;
-        }
-    }
-}
-
 // twiddles e^{-2 pi i q/P} read straight from the plan's FP64 table for Pmax
 struct StrideTw64 {
     const cplx<double>* p;

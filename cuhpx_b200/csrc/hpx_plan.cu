@@ -35,6 +35,7 @@
 
 #include "../../include/hpx_b200.h"
 #include "hpx_kernels.cuh"
+#include "legendre_direct.cuh"
 #include "legendre_tc.cuh"
 #include "hpx_remap.cuh"
 #include "hpx_healpy.cuh"
@@ -112,13 +113,14 @@ struct hpx_plan_s {
     int64_t Ftot = 0;        // complex spectrum entries per map over all rings
     int* d_lstart = nullptr;
     double2* d_pstart = nullptr;
-    int2* d_invwork = nullptr;
-    int n_invwork = 0;
     int Lpad = 0;                // coefficient row length (L + kCoefPad)
     double2* d_coef = nullptr;   // [M][Lpad] recurrence coefficients
     double2* d_seeds = nullptr;  // [M][seed_blocks(L)][2*nside] block seeds
     int2* d_fwdtiles = nullptr;  // (m, degree block) tiles of the forward contraction
     double* d_z = nullptr;       // cos(theta) of the north rings
+    RingLite* d_lite = nullptr;  // ring pairs as the direct contractions read them
+    double* d_alpha = nullptr;   // [M][Lpad] FP32 recurrence coefficients (legendre_direct.cuh)
+    double2* d_norm = nullptr;   // [M][Lpad] (c_l, 1 / c_l)
     AlphaC* d_alphac = nullptr;  // [M][Lpad] block-normalised recurrence (tensor-core producers)
     int* d_lsmax = nullptr;      // per order: max over its rings of the first significant degree
     std::vector<int> h_lsmax;
@@ -126,7 +128,7 @@ struct hpx_plan_s {
     float wmax = 0.f;            // largest ring weight w_t
     int ring_g = 16;             // maps per ring-FFT CTA (hpx_plan_set_schedule)
     int ring_streams = 2;        // 2: ring launches overlap on the aux stream; 1: serial
-    size_t ring_smem = 0, blue_smem = 0, blue3_smem = 0, fwd_smem = 0, inv_smem = 0;
+    size_t ring_smem = 0, blue_smem = 0, blue3_smem = 0, fwd_smem = 0;
     TcPlan tc;  // tensor-core contraction state (mixed precision plans)
 
     // per-kernel event timing (hpx_stats_*)
@@ -166,11 +168,13 @@ struct hpx_plan_s {
         cudaFree(d_chirp);
         cudaFree(d_lstart);
         cudaFree(d_pstart);
-        cudaFree(d_invwork);
         cudaFree(d_coef);
         cudaFree(d_seeds);
         cudaFree(d_fwdtiles);
         cudaFree(d_z);
+        cudaFree(d_lite);
+        cudaFree(d_alpha);
+        cudaFree(d_norm);
         cudaFree(d_alphac);
         cudaFree(d_lsmax);
         cudaFree(tc.d_err);
@@ -190,7 +194,8 @@ struct hpx_plan_s {
     size_t real_size() const { return f64 ? sizeof(double) : sizeof(float); }
     int cols() const { return ((2 * batch_chunk) + 3) & ~3; }
     size_t spec_bytes() const { return (size_t)M * 2 * NP * cols() * real_size(); }
-    size_t almT_bytes() const { return (size_t)M * L * cols() * real_size(); }
+    // order-major analysis output of the tensor cores where the ring spectra cannot hold it
+    size_t almT_bytes() const { return mixed() ? (size_t)M * L * cols() * real_size() : 0; }
     size_t resid_bytes() const { return (size_t)batch_chunk * npix * real_size(); }
     size_t F_bytes() const { return (size_t)batch_chunk * Ftot * 2 * real_size(); }
     bool mixed() const { return prec == HPX_PREC_BF16X3 || prec == HPX_PREC_F16X3; }
@@ -220,6 +225,28 @@ struct DeviceGuard {
         if (prev >= 0 && cur != prev) cudaSetDevice(prev);
     }
 };
+
+// largest L the plans accept
+template <typename T>
+constexpr int max_degrees() { return sizeof(T) == 4 ? 12956 : 11420; }
+
+// dynamic shared memory limits of the direct kernels (per function, as above)
+template <typename T, int C, int R>
+cudaError_t direct_attribute(int bytes) {
+    cudaError_t e = cudaFuncSetAttribute(k_leg_fwd_direct<T, C, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_leg_inv_direct<T, C, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes - 1024);
+}
+template <typename T>
+int direct_attributes(int dev_max) {
+    HPX_CUDA_TRY((direct_attribute<T, 2, 2>(dev_max)));
+    HPX_CUDA_TRY((direct_attribute<T, 2, 4>(dev_max)));
+    HPX_CUDA_TRY((direct_attribute<T, 4, 2>(dev_max)));
+    HPX_CUDA_TRY((direct_attribute<T, 4, 4>(dev_max)));
+    HPX_CUDA_TRY((direct_attribute<T, 8, 2>(dev_max)));
+    HPX_CUDA_TRY((direct_attribute<T, 8, sizeof(T) == 4 ? 4 : 2>(dev_max)));
+    return HPX_OK;
+}
 
 template <typename T>
 int create_typed(hpx_plan_s* P) {
@@ -278,12 +305,10 @@ int create_typed(hpx_plan_s* P) {
     P->blue3_smem =
         P->n_rings_blue3 ? (ring_smem_elems(P->bufP, P->nmax) + P->pblue3 / 2 + 2 + P->hblue3) * sizeof(C) : 0;
     P->fwd_smem = fwd_smem_bytes<T>();
-    P->inv_smem = inv_smem_bytes<T>(P->L);
     int dev_max = 0;
     HPX_CUDA_TRY(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device));
     if ((int)P->ring_smem > dev_max || (int)P->blue_smem > dev_max || (int)P->blue3_smem > dev_max ||
-        (int)P->fwd_smem > dev_max ||
-        (int)P->inv_smem > dev_max)
+        (int)P->fwd_smem > dev_max || P->L > max_degrees<T>())
         return set_err(HPX_ERR_UNSUPPORTED, "nside/lmax too large for the shared-memory kernels of this precision");
     // The attribute is per function, not per plan: always raise it to the device
     // maximum so that a plan needing less never lowers it under another plan.
@@ -296,10 +321,11 @@ int create_typed(hpx_plan_s* P) {
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_inv<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_inv<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_inv<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
+    const int rc_direct = direct_attributes<T>(dev_max);
+    if (rc_direct != HPX_OK) return rc_direct;
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_simt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_vleg_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_vleg_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_simt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     return HPX_OK;
 }
 
@@ -867,6 +893,13 @@ int plan_build(hpx_plan_s* P) {
         for (int p = 0; p < P->NP; ++p) hz[p] = P->h_pairs[p].z;
         HPX_CUDA_TRY(cudaMalloc(&P->d_z, sizeof(double) * P->NP));
         HPX_CUDA_TRY(cudaMemcpy(P->d_z, hz.data(), sizeof(double) * P->NP, cudaMemcpyHostToDevice));
+        std::vector<RingLite> lite(P->NP);
+        for (int p = 0; p < P->NP; ++p) {
+            const RingPair& rp = P->h_pairs[p];
+            lite[p] = RingLite{rp.foff_n, rp.has_south ? rp.foff_s : -1, rp.w, rp.h, rp.mt};
+        }
+        HPX_CUDA_TRY(cudaMalloc(&P->d_lite, sizeof(RingLite) * P->NP));
+        HPX_CUDA_TRY(cudaMemcpy(P->d_lite, lite.data(), sizeof(RingLite) * P->NP, cudaMemcpyHostToDevice));
         std::vector<int> hls((size_t)nms), hmax(P->M, 0);
         HPX_CUDA_TRY(cudaMemcpy(hls.data(), P->d_lstart, sizeof(int) * nms, cudaMemcpyDeviceToHost));
         for (int m = 0; m < P->M; ++m) {
@@ -886,6 +919,15 @@ int plan_build(hpx_plan_s* P) {
     {
         const int64_t n = (int64_t)P->M * P->Lpad;
         k_legendre_coef<<<(unsigned)((n + 255) / 256), 256>>>(P->M, P->L, P->Lpad, P->d_coef);
+        HPX_CUDA_TRY(cudaGetLastError());
+    }
+    if (!P->f64) {
+        const size_t n = (size_t)P->M * P->Lpad;
+        HPX_CUDA_TRY(cudaMalloc(&P->d_alpha, sizeof(double) * n));
+        HPX_CUDA_TRY(cudaMalloc(&P->d_norm, sizeof(double2) * n));
+        HPX_CUDA_TRY(cudaMemset(P->d_alpha, 0, sizeof(double) * n));
+        HPX_CUDA_TRY(cudaMemset(P->d_norm, 0, sizeof(double2) * n));
+        k_legendre_norm<<<(unsigned)((P->M + 31) / 32), 32>>>(P->M, P->L, P->Lpad, P->d_coef, P->d_alpha, P->d_norm);
         HPX_CUDA_TRY(cudaGetLastError());
     }
     HPX_CUDA_TRY(cudaMalloc(&P->d_alphac, sizeof(AlphaC) * (size_t)P->M * P->Lpad));
@@ -913,20 +955,6 @@ int plan_build(hpx_plan_s* P) {
         P->n_fwdtiles = (int)tiles.size();
         HPX_CUDA_TRY(cudaMalloc(&P->d_fwdtiles, sizeof(int2) * tiles.size()));
         HPX_CUDA_TRY(cudaMemcpy(P->d_fwdtiles, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice));
-    }
-
-    // ---- inverse work list: (m, ring block), heaviest first
-    std::vector<int2> work;
-    const int RBI = InvCfg<float>::RBI;
-    for (int m = 0; m < P->M; ++m) {
-        const int t0 = P->geo.first_ring(m);
-        const int K = P->NP - t0;
-        for (int rb = 0; rb < K; rb += RBI) work.push_back(make_int2(m, rb));
-    }
-    P->n_invwork = (int)work.size();
-    if (P->n_invwork > 0) {
-        HPX_CUDA_TRY(cudaMalloc(&P->d_invwork, sizeof(int2) * work.size()));
-        HPX_CUDA_TRY(cudaMemcpy(P->d_invwork, work.data(), sizeof(int2) * work.size(), cudaMemcpyHostToDevice));
     }
 
     int rc = P->f64 ? create_typed<double>(P) : create_typed<float>(P);
@@ -1050,8 +1078,8 @@ struct Pipeline {
         if (any_blue) blue(st);
     }
 
-    // map -> ring spectra F -> folded Legendre operand (spec, or bf16 hi/lo)
-    void ring_fwd(const T* map, int nb, int adjoint) {
+    // map -> ring spectra F
+    void ring_fft_fwd(const T* map, int nb, unsigned* fmax) {
         const int g = maps_per_cta_ring();
         {
             Timer tm(P, st, kStRingFwd);
@@ -1076,6 +1104,10 @@ struct Pipeline {
                             rt, P->rslot, gt, ch, fmax);
                 });
         }
+    }
+    // map -> ring spectra F -> folded Legendre operand (spec, or bf16 hi/lo)
+    void ring_fwd(const T* map, int nb, int adjoint) {
+        ring_fft_fwd(map, nb, fmax);
         Timer tm(P, st, kStFold);
         // |c (F_t +- F_t')| <= 2 max|c| max|F|: c = w_t, or c_m <= 2 for the adjoint
         fold_wb = adjoint ? 4.f : 2.f * P->wmax;
@@ -1090,6 +1122,10 @@ struct Pipeline {
             dim3 fg((P->mtmax + fold_mb<T>() - 1) / fold_mb<T>(), P->NP, (nb + 63) / 64);
             k_unfold<T><<<fg, 256, 0, st>>>(spec, P->cols(), nb, P->geo, P->d_pairs, adjoint, F, P->Ftot);
         }
+        ring_fft_inv(map, nb, ref);
+    }
+    // ring spectra F -> map
+    void ring_fft_inv(T* map, int nb, const T* ref) {
         const int g = maps_per_cta_ring();
         Timer tm(P, st, kStRingInv);
         const unsigned nbk = (nb + g - 1) / g;
@@ -1111,6 +1147,83 @@ struct Pipeline {
                         F, P->Ftot, map, nb, g, P->geo, P->d_pairs, P->d_rings + P->n_rings_pow2 + P->n_rings_blue,
                         rt, P->rslot, gt, ch, ref);
             });
+    }
+    // The contraction that reads and writes the ring spectra itself
+    // (legendre_direct.cuh): every FP32 and FP64 synthesis (nside 512, 64 maps:
+    // 4.6 ms against 6.3 ms of the tiled kernel it replaced, with its layout
+    // and unfold launches) and the analysis of up to 36 maps (FP32, nside 256: 32
+    // maps 708 us against 789 us tiled with the fold, 48 maps 987 against 878;
+    // FP64 crosses over there too: 32 maps 2003 against 1977 us).
+    bool direct_fwd(int nb) const { return !P->mixed() && nb <= (sizeof(T) == 4 ? 36 : 30); }
+    const typename DirRec<T>::Coef* dir_coef() const {
+        if constexpr (sizeof(T) == 4) return P->d_alpha;
+        else return P->d_coef;
+    }
+    template <int C, int R>
+    void leg_fwd_direct_launch(T* alm, int nb, int adjoint, int accumulate) {
+        const int gx = (P->M + kDirWarps - 1) / kDirWarps, gz = (nb + C / 2 - 1) / (C / 2);
+        // degrees per warp: long chunks amortise a ring's set-up, short ones
+        // give a small plan more warps
+        constexpr int lcap = 256, want = 4;  // (512 measured slower: fewer CTAs an SM)
+        int lch = kSeedBlock;
+        while (2 * lch <= lcap && lch < P->L && (int64_t)gx * gz * ((P->L + 2 * lch - 1) / (2 * lch)) >= want * 148) lch *= 2;
+        const int nch = (P->L + lch - 1) / lch;
+        const size_t sm = fwd_direct_smem<T, C, R>(lch);
+        k_leg_fwd_direct<T, C, R><<<dim3(nch + (accumulate ? 0 : 1), gx, gz), 32 * kDirWarps, sm, st>>>(
+            F, P->Ftot, nb, alm, P->L, P->M, P->geo, P->d_lite, P->d_z, P->d_lstart, P->d_pstart, dir_coef(), P->d_norm,
+            P->Lpad, P->d_seeds, lch, nch, adjoint, accumulate);
+    }
+    template <int C, int R>
+    void leg_inv_direct_launch(const T* alm, int nb, int adjoint) {
+        const dim3 grid((P->NP + 32 * R - 1) / (32 * R), (P->M + kDirWarps - 1) / kDirWarps, (nb + C / 2 - 1) / (C / 2));
+        k_leg_inv_direct<T, C, R><<<grid, 32 * kDirWarps, inv_direct_smem<T, C, R>(), st>>>(
+            alm, nb, F, P->Ftot, P->L, P->M, P->geo, P->d_lite, P->d_z, P->d_lstart, P->d_pstart, dir_coef(), P->d_norm,
+            P->Lpad, adjoint);
+    }
+    // Columns C: those of the map group, up to 8 (4 maps: beyond that the
+    // registers of the column values leave no room for R rings).  Rings R per
+    // lane: 4 (FP32 analysis at nside 1024, one map: 1566 us against 1836 with
+    // R = 2; synthesis 1327 against 1731), 2 where the wider FP64 columns would
+    // spill (C = 8: synthesis 58 us against 78 at nside 128, L = 511, 4 maps)
+    // and where R = 4 leaves a small plan too few warps: analysis with one block
+    // of 64 ring pairs (nside 32: 10.6 us against 12.4), synthesis below three
+    // CTAs an SM (nside 128, 8 maps: 30 us against 36).
+    void leg_fwd_direct(T* alm, int nb, int adjoint, int accumulate) {
+        Timer tm(P, st, kStLegFwd);
+        constexpr int R8 = sizeof(T) == 4 ? 4 : 2;
+        const bool small = P->NP <= 64;
+        if (nb == 1) small ? leg_fwd_direct_launch<2, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<2, 4>(alm, nb, adjoint, accumulate);
+        else if (nb == 2) small ? leg_fwd_direct_launch<4, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<4, 4>(alm, nb, adjoint, accumulate);
+        else small ? leg_fwd_direct_launch<8, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<8, R8>(alm, nb, adjoint, accumulate);
+    }
+    void leg_inv_direct(const T* alm, int nb, int adjoint) {
+        Timer tm(P, st, kStLegInv);
+        constexpr int R4 = sizeof(T) == 4 ? 4 : 2;
+        const int64_t ctas = (int64_t)((P->NP + 127) / 128) * ((P->M + kDirWarps - 1) / kDirWarps) * ((nb + 3) / 4);
+        const bool small = ctas < 3 * 148;
+        if (nb == 1) small ? leg_inv_direct_launch<2, 2>(alm, nb, adjoint) : leg_inv_direct_launch<2, 4>(alm, nb, adjoint);
+        else if (nb == 2) small ? leg_inv_direct_launch<4, 2>(alm, nb, adjoint) : leg_inv_direct_launch<4, R4>(alm, nb, adjoint);
+        else small ? leg_inv_direct_launch<8, 2>(alm, nb, adjoint) : leg_inv_direct_launch<8, R4>(alm, nb, adjoint);
+    }
+    // map -> alm (accumulate: added to alm)
+    void analysis(const T* map, T* alm, int nb, int adjoint, int accumulate) {
+        if (direct_fwd(nb)) {
+            ring_fft_fwd(map, nb, nullptr);
+            leg_fwd_direct(alm, nb, adjoint, accumulate);
+        } else {
+            ring_fwd(map, nb, adjoint);
+            leg_fwd(alm, nb, accumulate);
+        }
+    }
+    // alm -> map (ref: residual ref - map)
+    void synthesis(const T* alm, T* map, int nb, int adjoint, const T* ref) {
+        if (!P->mixed()) {
+            leg_inv_direct(alm, nb, adjoint);
+            ring_fft_inv(map, nb, ref);
+        } else {
+            leg_inv(alm, nb);
+            ring_inv(map, nb, adjoint, ref);
+        }
     }
     void leg_fwd(T* alm, int nb, int accumulate) {
         const int C = P->cols();
@@ -1146,48 +1259,34 @@ struct Pipeline {
     }
     void leg_inv(const T* alm, int nb) {
         const int C = P->cols();
-        if (P->mixed()) {
-            const TcPlan& TP = P->tc;
-            uint16_t* ah = tcA;
-            uint16_t* al = tcA + (size_t)2 * P->M * TP.Lh * kTcCols;
-            {
-                Timer tm(P, st, kStAlmCols);
-                if (amax) {
-                    cudaMemsetAsync(amax, 0, sizeof(unsigned) * nb, st);
-                    k_alm_maxabs<<<dim3((P->L + 7) / 8, nb), 256, 0, st>>>((const float*)alm, P->L, P->M, amax);
-                }
-                dim3 tg((P->M + 31) / 32, P->L + 64);
-                k_alm_to_tc<<<tg, dim3(32, 8), 0, st>>>((const float*)alm, nb, P->L, P->M, TP.Lh, ah, al, amax);
-            }
-            Timer tm(P, st, kStLegInv);
-            // orders the tensor cores do not visit must read as zero in the ring stage
-            if (TP.m_tc_end < P->M)
-                cudaMemsetAsync(spec + (size_t)TP.m_tc_end * 2 * P->NP * C, 0,
-                                (size_t)(P->M - TP.m_tc_end) * 2 * P->NP * C * sizeof(T), st);
-            if (TP.n_inv_tiles == 0) return;
-            CUtensorMap mh, ml;
-            if ((rc = encode_operand(P, &mh, ah, TP.Lh, 2ull * P->M, 32)) != HPX_OK) return;
-            if ((rc = encode_operand(P, &ml, al, TP.Lh, 2ull * P->M, 32)) != HPX_OK) return;
-            CUtensorMap sm = mh;
-            if (TP.table && (rc = encode_spec_store(P, &sm, spec)) != HPX_OK) return;
-            auto kern = TP.table ? (P->f16() ? k_leg_inv_tc<true, true> : k_leg_inv_tc<false, true>)
-                                 : (P->f16() ? k_leg_inv_tc<true, false> : k_leg_inv_tc<false, false>);
-            kern<<<TP.n_inv_ctas, kTcThreads, kISmem, st>>>(
-                mh, ml, TP.table ? TP.tab_inv : mh, sm, (float*)spec, C, nb, P->L, P->M, P->Lpad, P->geo, P->d_z, P->d_lstart, P->d_lsmax,
-                P->d_pstart, P->d_coef, P->d_alphac, P->d_seeds, TP.d_inv_tiles, TP.d_inv_off, amax, TP.d_err);
-            return;
-        }
-        dim3 tg((P->M + 31) / 32, P->L, (nb + 15) / 16);
+        const TcPlan& TP = P->tc;
+        uint16_t* ah = tcA;
+        uint16_t* al = tcA + (size_t)2 * P->M * TP.Lh * kTcCols;
         {
             Timer tm(P, st, kStAlmCols);
-            k_alm_to_cols<T><<<tg, dim3(32, 8), 0, st>>>(alm, nb, P->L, P->M, almT, C);
+            if (amax) {
+                cudaMemsetAsync(amax, 0, sizeof(unsigned) * nb, st);
+                k_alm_maxabs<<<dim3((P->L + 7) / 8, nb), 256, 0, st>>>((const float*)alm, P->L, P->M, amax);
+            }
+            dim3 tg((P->M + 31) / 32, P->L + 64);
+            k_alm_to_tc<<<tg, dim3(32, 8), 0, st>>>((const float*)alm, nb, P->L, P->M, TP.Lh, ah, al, amax);
         }
         Timer tm(P, st, kStLegInv);
-        if (P->n_invwork == 0) return;
-        dim3 grid(P->n_invwork, (C + InvCfg<T>::CT - 1) / InvCfg<T>::CT);
-        k_leg_inv_simt<T><<<grid, 256, P->inv_smem, st>>>(almT, C, spec, P->L, P->M, P->geo, P->d_pairs,
-                                                          P->d_lstart, P->d_pstart, P->d_coef, P->Lpad,
-                                                          P->d_invwork);
+        // orders the tensor cores do not visit must read as zero in the ring stage
+        if (TP.m_tc_end < P->M)
+            cudaMemsetAsync(spec + (size_t)TP.m_tc_end * 2 * P->NP * C, 0,
+                            (size_t)(P->M - TP.m_tc_end) * 2 * P->NP * C * sizeof(T), st);
+        if (TP.n_inv_tiles == 0) return;
+        CUtensorMap mh, ml;
+        if ((rc = encode_operand(P, &mh, ah, TP.Lh, 2ull * P->M, 32)) != HPX_OK) return;
+        if ((rc = encode_operand(P, &ml, al, TP.Lh, 2ull * P->M, 32)) != HPX_OK) return;
+        CUtensorMap sm = mh;
+        if (TP.table && (rc = encode_spec_store(P, &sm, spec)) != HPX_OK) return;
+        auto kern = TP.table ? (P->f16() ? k_leg_inv_tc<true, true> : k_leg_inv_tc<false, true>)
+                             : (P->f16() ? k_leg_inv_tc<true, false> : k_leg_inv_tc<false, false>);
+        kern<<<TP.n_inv_ctas, kTcThreads, kISmem, st>>>(
+            mh, ml, TP.table ? TP.tab_inv : mh, sm, (float*)spec, C, nb, P->L, P->M, P->Lpad, P->geo, P->d_z, P->d_lstart, P->d_lsmax,
+            P->d_pstart, P->d_coef, P->d_alphac, P->d_seeds, TP.d_inv_tiles, TP.d_inv_off, amax, TP.d_err);
     }
 };
 
@@ -1300,21 +1399,17 @@ int run_op(hpx_plan_s* P, Op op, const void* in, void* out, int64_t batch, void*
             case kInverseAdjoint: {
                 const T* map = (const T*)in + b0 * P->npix;
                 T* alm = (T*)out + b0 * alm_stride;
-                pl.ring_fwd(map, nb, op == kForward ? 0 : 1);
-                pl.leg_fwd(alm, nb, 0);
+                pl.analysis(map, alm, nb, op == kForward ? 0 : 1, 0);
                 break;
             }
             case kForwardRefined: {
                 // a = S f;  repeat: r = f - I a;  a += S r
                 const T* map = (const T*)in + b0 * P->npix;
                 T* alm = (T*)out + b0 * alm_stride;
-                pl.ring_fwd(map, nb, 0);
-                pl.leg_fwd(alm, nb, 0);
+                pl.analysis(map, alm, nb, 0, 0);
                 for (int it = 0; it < iters; ++it) {
-                    pl.leg_inv(alm, nb);
-                    pl.ring_inv(pl.resid, nb, 0, map);
-                    pl.ring_fwd(pl.resid, nb, 0);
-                    pl.leg_fwd(alm, nb, 1);
+                    pl.synthesis(alm, pl.resid, nb, 0, map);
+                    pl.analysis(pl.resid, alm, nb, 0, 1);
                 }
                 break;
             }
@@ -1322,8 +1417,7 @@ int run_op(hpx_plan_s* P, Op op, const void* in, void* out, int64_t batch, void*
             case kForwardAdjoint: {
                 const T* alm = (const T*)in + b0 * alm_stride;
                 T* map = (T*)out + b0 * P->npix;
-                pl.leg_inv(alm, nb);
-                pl.ring_inv(map, nb, op == kInverse ? 0 : 1, nullptr);
+                pl.synthesis(alm, map, nb, op == kInverse ? 0 : 1, nullptr);
                 break;
             }
         }
@@ -1445,8 +1539,7 @@ int run_forward_noalloc(hpx_plan_s* P, const void* in, void* out, int64_t batch,
     for (int64_t b0 = 0; b0 < batch; b0 += bc) {
         const int nb = (int)std::min<int64_t>(bc, batch - b0);
         set_extents(P, st, (int64_t)nb * P->npix, (int64_t)nb * alm_stride, nb);
-        pl.ring_fwd((const T*)in + b0 * P->npix, nb, 0);
-        pl.leg_fwd((T*)out + b0 * alm_stride, nb, 0);
+        pl.analysis((const T*)in + b0 * P->npix, (T*)out + b0 * alm_stride, nb, 0, 0);
         if (pl.rc != HPX_OK) return pl.rc;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return set_err(HPX_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));

@@ -1,4 +1,5 @@
-// Associated-Legendre recurrence and the SIMT Legendre contractions.
+// Associated-Legendre recurrence and the tiled SIMT analysis contraction (the
+// synthesis and the analysis of few maps are in legendre_direct.cuh).
 //
 // Pbar_l^m(x) is the orthonormal associated Legendre function without the
 // Condon-Shortley phase, as built by legpoly / legpoly_torch
@@ -362,144 +363,6 @@ __global__ void __launch_bounds__(256) k_leg_fwd_simt(const T* __restrict__ spec
                 cplx<T> v = {acc[i][cc], acc[i][cc + 1]};
                 if (accumulate) v = cadd(*dst, v);
                 *dst = v;
-            }
-        }
-    }
-}
-
-// ------------------------------------------------------------ inverse (synthesis)
-// E[m][p][c] = sum_{l-m even} Pbar_l^m(x_p) A[m][l][c],  O = sum over l-m odd,
-// written to spec[m][0][p][c] and spec[m][1][p][c].  One CTA per (m, block of
-// RBI rings, column tile); the FP64 recurrence of each ring runs in one thread.
-template <typename T>
-struct InvCfg {
-    static constexpr int RBI = 64;  // rings per CTA
-    static constexpr int CT = 128;  // columns per CTA
-    static constexpr int LC = 32;   // degrees per staged chunk
-    static constexpr int RBP = RBI + 16 / sizeof(T);
-};
-
-template <typename T>
-__host__ __device__ constexpr size_t inv_smem_bytes(int L) {
-    using C = InvCfg<T>;
-    return (size_t)2 * L * sizeof(double) + (size_t)C::LC * C::RBP * sizeof(T) + (size_t)C::LC * C::CT * sizeof(T) + 64;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_leg_inv_simt(const T* __restrict__ almT, int C, T* __restrict__ spec, int L,
-                                                      int M, Geom geo, const RingPair* __restrict__ pairs,
-                                                      const int* __restrict__ lstart,
-                                                      const double2* __restrict__ pstart,
-                                                      const double2* __restrict__ coef, int Lpad,
-                                                      const int2* __restrict__ work) {
-    using Cfg = InvCfg<T>;
-    constexpr int RBI = Cfg::RBI, CT = Cfg::CT, LC = Cfg::LC, RBP = Cfg::RBP;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int NP = geo.NP;
-    const int2 wk = work[blockIdx.x];
-    const int m = wk.x, rb = wk.y;
-    const int c0 = blockIdx.y * CT;
-    const int tid = threadIdx.x;
-    double* coefA = (double*)smem_raw;
-    double* coefB = coefA + L;
-    T* Pt = (T*)(coefB + L);  // [LC][RBP], 16-byte aligned (2L doubles precede it)
-    T* As = Pt + LC * RBP;                                          // [LC][CT]
-
-    const int t0 = geo.first_ring(m);
-    const int K = NP - t0;
-
-    for (int l = m + 2 + tid; l < L; l += blockDim.x) {
-        const double2 ab = coef[(int64_t)m * Lpad + l];
-        coefA[l] = ab.x;
-        coefB[l] = ab.y;
-    }
-    // generator state (threads tid < RBI own ring rb + tid)
-    const int rg = rb + tid;
-    const bool gen = tid < RBI && rg < K;
-    double x = 0.0, p1 = 0.0, p2 = 0.0;
-    int ls = L;
-    double2 ps = make_double2(0.0, 0.0);
-    if (gen) {
-        x = pairs[t0 + rg].z;
-        ls = lstart[(int64_t)m * NP + t0 + rg];
-        if (ls < L) ps = pstart[(int64_t)m * NP + t0 + rg];
-    }
-    __syncthreads();
-
-    const int tx = tid & 15, ty = tid >> 4;
-    const int rrow = ty * 4;
-    const int cA = tx * 4, cB = 64 + tx * 4;
-    T accE[4][8], accO[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            accE[i][c] = (T)0;
-            accO[i][c] = (T)0;
-        }
-
-    for (int l0 = m; l0 < L; l0 += LC) {
-        if (tid < RBI) {
-            for (int i = 0; i < LC; ++i) {
-                const int l = l0 + i;
-                double v = 0.0;
-                if (gen && l < L) v = leg_step(l, ls, ps, l >= m + 2 ? coefA[l] : 0.0, l >= m + 2 ? coefB[l] : 0.0, x, p1, p2);
-                p2 = p1;
-                p1 = v;
-                Pt[i * RBP + tid] = (T)v;
-            }
-        }
-        for (int i = tid; i < LC * CT; i += blockDim.x) {
-            const int c = i % CT, li = i / CT;
-            const int l = l0 + li;
-            T v = (T)0;
-            if (l < L && c0 + c < C) v = almT[((int64_t)m * L + l) * C + c0 + c];
-            As[li * CT + c] = v;
-        }
-        __syncthreads();
-#pragma unroll 2
-        for (int li = 0; li < LC; li += 2) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const T* pr = Pt + (li + h) * RBP + rrow;
-                const T* ar = As + (li + h) * CT;
-                T pv[4], av[8];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) pv[i] = pr[i];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    av[c] = ar[cA + c];
-                    av[4 + c] = ar[cB + c];
-                }
-                if (h == 0) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) accE[i][c] = fma(pv[i], av[c], accE[i][c]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) accO[i][c] = fma(pv[i], av[c], accO[i][c]);
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // write E/O for rings of this CTA
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = rb + rrow + i;
-        if (r >= K || !HPX_INB((((int64_t)m * 2 + 1) * NP + t0 + r) * C + c0 + min(CT, C - c0) - 1, kExtSpec, 16))
-            continue;
-        T* e = spec + (((int64_t)m * 2 + 0) * NP + t0 + r) * C + c0;
-        T* o = spec + (((int64_t)m * 2 + 1) * NP + t0 + r) * C + c0;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const int cc = c < 4 ? cA + c : cB + c - 4;
-            if (c0 + cc < C) {
-                e[cc] = accE[i][c];
-                o[cc] = accO[i][c];
             }
         }
     }
