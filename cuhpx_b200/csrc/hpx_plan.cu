@@ -237,8 +237,18 @@ cudaError_t direct_attribute(int bytes) {
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_leg_inv_direct<T, C, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes - 1024);
 }
+template <typename T, int CV, int R>
+cudaError_t vec_attribute(int bytes) {
+    cudaError_t e = cudaFuncSetAttribute(k_vleg_fwd<T, CV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_vleg_inv<T, CV, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes - 1024);
+}
 template <typename T>
 int direct_attributes(int dev_max) {
+    HPX_CUDA_TRY((vec_attribute<T, 1, 2>(dev_max)));
+    HPX_CUDA_TRY((vec_attribute<T, 1, 4>(dev_max)));
+    HPX_CUDA_TRY((vec_attribute<T, 2, 2>(dev_max)));
+    HPX_CUDA_TRY((vec_attribute<T, 2, sizeof(T) == 4 ? 4 : 2>(dev_max)));
     HPX_CUDA_TRY((direct_attribute<T, 2, 2>(dev_max)));
     HPX_CUDA_TRY((direct_attribute<T, 2, 4>(dev_max)));
     HPX_CUDA_TRY((direct_attribute<T, 4, 2>(dev_max)));
@@ -324,8 +334,6 @@ int create_typed(hpx_plan_s* P) {
     const int rc_direct = direct_attributes<T>(dev_max);
     if (rc_direct != HPX_OK) return rc_direct;
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_simt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_vleg_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_vleg_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     return HPX_OK;
 }
 
@@ -896,7 +904,8 @@ int plan_build(hpx_plan_s* P) {
         std::vector<RingLite> lite(P->NP);
         for (int p = 0; p < P->NP; ++p) {
             const RingPair& rp = P->h_pairs[p];
-            lite[p] = RingLite{rp.foff_n, rp.has_south ? rp.foff_s : -1, rp.w, rp.h, rp.mt};
+            lite[p] = RingLite{rp.foff_n, rp.has_south ? rp.foff_s : -1, rp.w, rp.h, rp.mt,
+                               rp.s2 > 0.0 ? 1.0 / std::sqrt(rp.s2) : 0.0, 0.0};
         }
         HPX_CUDA_TRY(cudaMalloc(&P->d_lite, sizeof(RingLite) * P->NP));
         HPX_CUDA_TRY(cudaMemcpy(P->d_lite, lite.data(), sizeof(RingLite) * P->NP, cudaMemcpyHostToDevice));
@@ -1159,14 +1168,18 @@ struct Pipeline {
         if constexpr (sizeof(T) == 4) return P->d_alpha;
         else return P->d_coef;
     }
+    // Degrees per warp of an analysis: long chunks amortise a ring block's set-up,
+    // short ones give a small plan more CTAs (`groups` CTAs per chunk; four an SM
+    // wanted).  512 measured slower than 256 (fewer CTAs fit an SM).
+    static int degree_chunk(int L, int64_t groups) {
+        int lch = kSeedBlock;
+        while (2 * lch <= 256 && lch < L && groups * ((L + 2 * lch - 1) / (2 * lch)) >= 4 * 148) lch *= 2;
+        return lch;
+    }
     template <int C, int R>
     void leg_fwd_direct_launch(T* alm, int nb, int adjoint, int accumulate) {
         const int gx = (P->M + kDirWarps - 1) / kDirWarps, gz = (nb + C / 2 - 1) / (C / 2);
-        // degrees per warp: long chunks amortise a ring's set-up, short ones
-        // give a small plan more warps
-        constexpr int lcap = 256, want = 4;  // (512 measured slower: fewer CTAs an SM)
-        int lch = kSeedBlock;
-        while (2 * lch <= lcap && lch < P->L && (int64_t)gx * gz * ((P->L + 2 * lch - 1) / (2 * lch)) >= want * 148) lch *= 2;
+        const int lch = degree_chunk(P->L, gx * gz);
         const int nch = (P->L + lch - 1) / lch;
         const size_t sm = fwd_direct_smem<T, C, R>(lch);
         k_leg_fwd_direct<T, C, R><<<dim3(nch + (accumulate ? 0 : 1), gx, gz), 32 * kDirWarps, sm, st>>>(
@@ -1204,6 +1217,42 @@ struct Pipeline {
         if (nb == 1) small ? leg_inv_direct_launch<2, 2>(alm, nb, adjoint) : leg_inv_direct_launch<2, 4>(alm, nb, adjoint);
         else if (nb == 2) small ? leg_inv_direct_launch<4, 2>(alm, nb, adjoint) : leg_inv_direct_launch<4, R4>(alm, nb, adjoint);
         else small ? leg_inv_direct_launch<8, 2>(alm, nb, adjoint) : leg_inv_direct_launch<8, R4>(alm, nb, adjoint);
+    }
+    // spin-1 contractions (vector.cuh) of a plan with one more degree and order
+    template <int CV, int R>
+    void vleg_fwd_launch(T* alm, int nb, int csphase, int adjoint, int use_nf) {
+        const int Lv = P->L - 1, Mv = P->M - 1;
+        const int gx = (Mv + kDirWarps - 1) / kDirWarps, gz = (nb + CV - 1) / CV;
+        const int lch = degree_chunk(Lv, gx * gz);
+        const int nch = (Lv + lch - 1) / lch;
+        k_vleg_fwd<T, CV, R><<<dim3(nch + 1, gx, gz), 32 * kDirWarps, vfwd_smem_bytes<T, CV, R>(lch), st>>>(
+            F, P->Ftot, nb, alm, Lv, Mv, P->L, P->geo, P->d_lite, P->d_z, P->d_lstart, P->d_pstart, dir_coef(),
+            P->d_norm, P->Lpad, P->d_seeds, lch, nch, csphase, adjoint, use_nf);
+    }
+    template <int CV, int R>
+    void vleg_inv_launch(const T* alm, int nb, int csphase, int adjoint, int use_nf) {
+        const dim3 grid((P->NP + 32 * R - 1) / (32 * R), (P->M + kDirWarps - 1) / kDirWarps, (nb + CV - 1) / CV);
+        k_vleg_inv<T, CV, R><<<grid, 32 * kDirWarps, vinv_smem_bytes<T, CV, R>(), st>>>(
+            alm, nb, F, P->Ftot, P->L - 1, P->M - 1, P->L, P->M, P->geo, P->d_lite, P->d_z, P->d_lstart, P->d_pstart,
+            dir_coef(), P->d_norm, P->Lpad, P->d_seeds, csphase, adjoint, use_nf);
+    }
+    // Two vector maps at a time (8 columns of each kind) and R as for the scalar
+    // contractions (nside 256, 16 maps, FP32: analysis 1208 us with R = 4, 1719
+    // with 2; nside 128, 4 maps, synthesis 60 against 48 us: too few CTAs with 4).
+    void vleg_fwd(T* alm, int nb, int csphase, int adjoint, int use_nf) {
+        Timer tm(P, st, kStLegFwd);
+        constexpr int R2 = sizeof(T) == 4 ? 4 : 2;
+        const bool small = P->NP <= 64;
+        if (nb == 1) small ? vleg_fwd_launch<1, 2>(alm, nb, csphase, adjoint, use_nf) : vleg_fwd_launch<1, 4>(alm, nb, csphase, adjoint, use_nf);
+        else small ? vleg_fwd_launch<2, 2>(alm, nb, csphase, adjoint, use_nf) : vleg_fwd_launch<2, R2>(alm, nb, csphase, adjoint, use_nf);
+    }
+    void vleg_inv(const T* alm, int nb, int csphase, int adjoint, int use_nf) {
+        Timer tm(P, st, kStLegInv);
+        constexpr int R4 = sizeof(T) == 4 ? 4 : 2;
+        const int64_t ctas = (int64_t)((P->NP + 127) / 128) * ((P->M + kDirWarps - 1) / kDirWarps) * ((nb + 1) / 2);
+        const bool small = ctas < 3 * 148;
+        if (nb == 1) small ? vleg_inv_launch<1, 2>(alm, nb, csphase, adjoint, use_nf) : vleg_inv_launch<1, R4>(alm, nb, csphase, adjoint, use_nf);
+        else small ? vleg_inv_launch<2, 2>(alm, nb, csphase, adjoint, use_nf) : vleg_inv_launch<2, R4>(alm, nb, csphase, adjoint, use_nf);
     }
     // map -> alm (accumulate: added to alm)
     void analysis(const T* map, T* alm, int nb, int adjoint, int accumulate) {
@@ -1329,7 +1378,6 @@ template <typename T>
 int run_vec(hpx_plan_s* P, Op op, const void* in, void* out, int64_t batch, void* ws, cudaStream_t st, int csphase) {
     Pipeline<T> pl(P, ws, st);
     const int Lv = P->L - 1, Mv = P->M - 1;
-    const int C = P->cols();
     const int64_t vc = std::max(1, P->batch_chunk / 2);
     const size_t alm_stride = (size_t)2 * Lv * Mv * 2;
     const size_t map_stride = (size_t)2 * P->npix;
@@ -1340,26 +1388,13 @@ int run_vec(hpx_plan_s* P, Op op, const void* in, void* out, int64_t batch, void
         if (analysis) {
             const T* map = (const T*)in + b0 * map_stride;
             T* alm = (T*)out + b0 * alm_stride;
-            pl.ring_fwd(map, 2 * nb, op == kForward ? 0 : 1);
-            typename Pipeline<T>::Timer tm(P, st, kStLegFwd);
-            const int nj = (Lv + VFwdCfg<T>::LT - 1) / VFwdCfg<T>::LT;
-            const dim3 grid((unsigned)(Mv * nj), (unsigned)((C + VFwdCfg<T>::CT - 1) / VFwdCfg<T>::CT));
-            k_vleg_fwd<T><<<grid, 256, vfwd_smem_bytes<T>(), st>>>(
-                pl.spec, C, nb, alm, Lv, Mv, P->L, P->M, P->Lpad, P->geo, P->d_pairs, P->d_lstart, P->d_pstart,
-                P->d_coef, P->d_seeds, csphase, op == kForward ? 1 : 0);
+            pl.ring_fft_fwd(map, 2 * nb, nullptr);
+            pl.vleg_fwd(alm, nb, csphase, op == kForward ? 0 : 1, op == kForward ? 1 : 0);
         } else {
             const T* alm = (const T*)in + b0 * alm_stride;
             T* map = (T*)out + b0 * map_stride;
-            {
-                typename Pipeline<T>::Timer tm(P, st, kStLegInv);
-                const int nr = (P->NP + VInvCfg<T>::RBI - 1) / VInvCfg<T>::RBI;
-                const dim3 grid((unsigned)(P->M * nr), (unsigned)((C + VInvCfg<T>::CT - 1) / VInvCfg<T>::CT));
-                k_vleg_inv<T><<<grid, 256, vinv_smem_bytes<T>(), st>>>(alm, nb, pl.spec, C, Lv, Mv, P->L, P->M,
-                                                                       P->Lpad, P->geo, P->d_pairs, P->d_lstart,
-                                                                       P->d_pstart, P->d_coef, csphase,
-                                                                       op == kForwardAdjoint ? 1 : 0);
-            }
-            pl.ring_inv(map, 2 * nb, op == kInverse ? 0 : 1, nullptr);
+            pl.vleg_inv(alm, nb, csphase, op == kForwardAdjoint ? 1 : 0, op == kForwardAdjoint ? 1 : 0);
+            pl.ring_fft_inv(map, 2 * nb, nullptr);
         }
         if (pl.rc != HPX_OK) return pl.rc;
         cudaError_t e = cudaGetLastError();

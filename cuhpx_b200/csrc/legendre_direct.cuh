@@ -95,12 +95,14 @@ constexpr int kDirWarps = 4;   // orders per CTA: 4 consecutive FP32 spectra ent
 constexpr int kDirChunk = 32;  // degrees per staged coefficient chunk (synthesis)
 constexpr int kNoDegree = 0x3fffffff;
 
-// What the direct kernels need to know about a ring pair (32 bytes; RingPair is
-// four times that, and its fields would be gathered one sector each)
+// What the direct kernels need to know about a ring pair (48 bytes; RingPair is
+// almost three times that, and its fields would be gathered one sector each)
 struct __align__(16) RingLite {
     int64_t foff_n, foff_s;  // spectrum offsets; foff_s < 0: no south ring
     double w;
     int h, mt;
+    double rs;  // 1 / sin(theta), 0 at a pole
+    double pad;
 };
 
 // Recurrence in the form each precision uses.

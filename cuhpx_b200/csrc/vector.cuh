@@ -14,421 +14,615 @@
 // and the synthesis of ring spectra (s, t) of the two components:
 //   s_tm = sum_l (D0 S + i D1 T)              t_tm = sum_l (-D0 T + i D1 S).
 // The reference tabulates D0, D1 densely ([2][M][L][rings], FP64) and runs
-// eight einsums per call; here they are generated on the fly from FP64
-// recurrences of orders m-1 and m+1, which the plan provides because the
-// vector plan is built with L+1 degrees and M+1 orders.
+// eight einsums per call.  Here they are generated on the fly:
+//
+//   FP32  from the one recurrence of order m that the scalar kernels run: D0 is
+//         dPbar/dtheta and D1 is m Pbar / sin(theta), so
+//           sin(theta) D0_l = f_l Pbar_{l+1} - (l+1) x Pbar_l,
+//           f_l = sqrt((2l+1)/(2l+3) ((l+1)^2 - m^2)),    sin(theta) D1_l = m Pbar_l
+//         with the pair (Pbar_l, Pbar_{l+1}) the recurrence carries anyway;
+//         1/sin(theta) goes into the folded spectra or onto the finished ring
+//         sums.  The subtraction, in FP64, loses a factor 1/sin(theta) next to
+//         the poles: nothing FP32 values notice (errors against FP64 measured 10
+//         to 40% below the form with two recurrences), but
+//   FP64  would (3e-14 against 5e-15 in maps at nside 256), so it runs the
+//         recurrences of orders m-1 and m+1 (two more operations a value beside the
+//         16 of the products).
+// The vector plan is built with L+1 degrees and M+1 orders for them.
 //
 // North/south symmetry: Pbar_l^m(-x) = (-1)^{l+m} Pbar_l^m(x), so D0 has the
 // parity (-1)^{l+m+1} and D1 the parity (-1)^{l+m}: the analysis contracts D0
 // with the fold of parity index (l-m+1)&1 and D1 with (l-m)&1 (S = w(F_t +
 // F_t'), D = w(F_t - F_t')); the synthesis sums the terms whose south sign is +
-// into E and the others into O, so that the scalar path's unfold (F_t = E + O,
-// F_t' = E - O) and inverse ring FFTs finish the job.  The two components of
-// every vector map travel through the ring stages as two consecutive maps.
+// into E and the others into O (F_t = E + O, F_t' = E - O).  The two components
+// of every vector map travel through the ring FFTs as two consecutive maps.
+//
+// The kernels are those of legendre_direct.cuh with two values and eight columns
+// per vector map: a warp per order, 32 R rings by lane, nothing tabulated and no
+// fold or unfold launch.  The tiled kernels before
+// them ran recurrences of orders m-1 and m+1 and 64 columns whatever the batch:
+// analysis + synthesis of 4 maps at nside 128, L = M = 255, FP32 1282 -> 158 us.
 #pragma once
 
-#include "legendre.cuh"
+#include "legendre_direct.cuh"
 
 namespace hpx {
 
-// Running FP64 recurrence of one order o at one ring: value at degree d,
-// stepping upward; degrees below o (and below the first significant degree)
-// read as zero.
-struct LegRun {
-    int o, d, ls;
-    double2 ps;
-    double x, p1, p2;
-    __device__ void init(int order, int m_end, int M, int64_t mi, const int* __restrict__ lstart,
-                         const double2* __restrict__ pstart, double xv) {
-        o = order;
-        d = order;
-        x = xv;
-        p1 = p2 = 0.0;
-        ls = (order < m_end) ? lstart[mi] : 0x7fffffff;
-        ps = (order < m_end && ls < 0x7fffffff) ? pstart[mi] : make_double2(0.0, 0.0);
-        (void)M;
+// Factors of degree l: FP32 f_l c_{l+1} / c_l and l + 1; FP64 those of the four
+// terms of D0 and D1
+template <typename T>
+struct VecFac;
+template <>
+struct VecFac<float> {
+    double f, lp;
+    static __device__ __forceinline__ VecFac make(int l, int m, const double2* __restrict__ nm, int Lv) {
+        if (l >= Lv) return {0.0, 0.0};
+        const double dl = l;
+        const double f = sqrt((2.0 * dl + 1.0) / (2.0 * dl + 3.0) * ((dl + 1.0 - m) * (dl + 1.0 + m)));
+        return {f * nm[l + 1].x * nm[l].y, dl + 1.0};
     }
-    // value at degree d, then d += 1
-    __device__ double next(const double2* __restrict__ coef_o, int Lp) {
-        double v = 0.0;
-        if (d < Lp) {
-            const double2 ab = d >= o + 2 ? coef_o[d] : make_double2(0.0, 0.0);
-            v = leg_step(d, ls, ps, ab.x, ab.y, x, p1, p2);
-        }
-        p2 = p1;
-        p1 = v;
-        ++d;
-        return v;
+};
+template <>
+struct VecFac<double> {
+    double c1, c2, c3, c4;
+    static __device__ __forceinline__ VecFac make(int l, int m, const double2* __restrict__, int Lv) {
+        if (l >= Lv || l < m) return {0.0, 0.0, 0.0, 0.0};
+        const double dl = l, dm = m;
+        const double h = 0.5 * sqrt((2.0 * dl + 1.0) / (2.0 * dl + 3.0));
+        return {0.5 * sqrt((dl + dm) * (dl - dm + 1.0)), 0.5 * sqrt((dl - dm) * (dl + dm + 1.0)),
+                m ? h * sqrt((dl - dm + 1.0) * (dl - dm + 2.0)) : 0.0, m ? h * sqrt((dl + dm + 1.0) * (dl + dm + 2.0)) : 0.0};
     }
 };
 
-// 0.5 sqrt(...) factors of D0 and D1 at (l, m)
-__device__ __forceinline__ void vec_coefs(int l, int m, double& c1, double& c2, double& c3, double& c4) {
-    const double dl = l, dm = m;
-    c1 = 0.5 * sqrt((dl + dm) * (dl - dm + 1.0));
-    c2 = 0.5 * sqrt((dl - dm) * (dl + dm + 1.0));
-    const double h = 0.5 * sqrt((2.0 * dl + 1.0) / (2.0 * dl + 3.0));
-    c3 = h * sqrt((dl - dm + 1.0) * (dl - dm + 2.0));
-    c4 = h * sqrt((dl + dm + 1.0) * (dl + dm + 2.0));
+// One ring's generator at degree l: the values p0 ~ D0_l, p1 ~ D1_l (FP32: times
+// sin(theta) / c_l, and 1 / m for p1).  start(l) must be called before value() at
+// every degree at which a recurrence may start.
+template <typename T>
+struct VecGen;
+template <>
+struct VecGen<float> {
+    static constexpr bool kScaled = true;  // 1/sin(theta) and m are applied elsewhere
+    int ls;
+    double x, u0, u1;
+    struct Order {
+        const double* coef;  // alpha of degree l + 2 at [l]
+        const double2* nm;
+        int64_t row;  // m * NP
+        int m, L;
+    };
+    static __device__ __forceinline__ Order order(int m, int, int Lp, int Lpad, int NP, const double* coef,
+                                                  const double2* norm) {
+        return {coef + (int64_t)m * Lpad + 2, norm + (int64_t)m * Lpad, (int64_t)m * NP, m, Lp};
+    }
+    __device__ __forceinline__ void clear() {
+        ls = kNoDegree;
+        x = u0 = u1 = 0.0;
+    }
+    // first degree (from l0 on) that can be nonzero, kNoDegree if none below lend
+    __device__ __forceinline__ int init(const Order& o, int p, double z, int l0, int lend,
+                                        const int* __restrict__ lstart) {
+        x = z;
+        const int s = lstart[o.row + p];
+        if (s < lend) ls = s;
+        return ls;
+    }
+    // the pair at l0 (= m + a multiple of 64) from the block seeds
+    __device__ __forceinline__ void seed(const Order& o, int p, int NP, int l0, const double2* __restrict__ seeds,
+                                         const double2* __restrict__) {
+        if (ls <= l0) {
+            const double2 sd =
+                dir_start<float>(seeds[((int64_t)o.m * seed_blocks(o.L) + (l0 - o.m) / kSeedBlock) * NP + p], o.nm, l0, o.L);
+            u0 = sd.x;
+            u1 = sd.y;
+            ls = l0 - 1;  // started
+        }
+    }
+    __device__ __forceinline__ int last_start(int l0) const { return ls >= l0 && ls < kNoDegree ? ls : -1; }
+    __device__ __forceinline__ void start(const Order& o, int p, int l, const double2* __restrict__ pstart) {
+        if (ls == l) {
+            const double2 ps = dir_start<float>(pstart[o.row + p], o.nm, l, o.L);
+            u0 = ps.x;
+            u1 = ps.y;
+        }
+    }
+    struct Coef {
+        double al;
+    };
+    static __device__ __forceinline__ Coef load(const Order& o, int l) { return {o.coef[l]}; }
+    __device__ __forceinline__ void value(const VecFac<float>& f, int, float& p0, float& p1) const {
+        p0 = (float)fma(f.f, u1, -(f.lp * x) * u0);
+        p1 = (float)u0;
+    }
+    __device__ __forceinline__ void advance(const Coef& c) { DirRec<float>::advance(c.al, x, u0, u1); }
+};
+template <>
+struct VecGen<double> {
+    static constexpr bool kScaled = false;
+    int la, lb;                   // starts of orders m - 1 and m + 1
+    double x, a0, a1, b0, b1;     // their pairs at l, l + 1
+    struct Order {
+        const double2 *ca, *cb;
+        int64_t ra, rb;
+        int m, L;
+    };
+    static __device__ __forceinline__ Order order(int m, int Mp, int Lp, int Lpad, int NP, const double2* coef,
+                                                  const double2*) {
+        const int ma = m ? m - 1 : 0, mb = min(m + 1, Mp - 1);  // (m < Mv = Mp - 1 wherever values are used)
+        return {coef + (int64_t)ma * Lpad + 2, coef + (int64_t)mb * Lpad + 2, (int64_t)ma * NP, (int64_t)mb * NP, m, Lp};
+    }
+    __device__ __forceinline__ void clear() {
+        la = lb = kNoDegree;
+        x = a0 = a1 = b0 = b1 = 0.0;
+    }
+    __device__ __forceinline__ int init(const Order& o, int p, double z, int l0, int lend,
+                                        const int* __restrict__ lstart) {
+        x = z;
+        // a value of degree l also takes the pairs' second elements: one degree earlier
+        const int sb = lstart[o.rb + p];
+        if (sb <= lend) lb = sb;
+        if (o.m) {
+            const int sa = lstart[o.ra + p];
+            if (sa <= lend) la = sa;
+        }
+        const int s = min(la, lb);
+        return s == kNoDegree ? s : max(s - 1, l0);
+    }
+    __device__ __forceinline__ void seed(const Order& o, int p, int NP, int l0, const double2* __restrict__ seeds,
+                                         const double2* __restrict__ pstart) {
+        const int j = (l0 - o.m) / kSeedBlock, nb = seed_blocks(o.L);
+        if (la < l0) {  // order m - 1: block j starts at l0 - 1
+            const double2 sd = seeds[((int64_t)(o.m - 1) * nb + j) * NP + p];
+            a0 = sd.x;
+            a1 = sd.y;
+            DirRec<double>::advance(o.ca[l0 - 1], x, a0, a1);
+        }
+        if (j > 0 && lb < l0) {  // order m + 1: block j - 1 starts at l0 - 63
+            const int l1 = l0 + 1 - kSeedBlock;
+            if (lb <= l1) {
+                const double2 sd = seeds[((int64_t)(o.m + 1) * nb + j - 1) * NP + p];
+                b0 = sd.x;
+                b1 = sd.y;
+            }
+#pragma unroll 1
+            for (int l = l1; l < l0; ++l) {
+                if (lb == l && lb > l1) {
+                    const double2 ps = pstart[o.rb + p];
+                    b0 = ps.x;
+                    b1 = ps.y;
+                }
+                DirRec<double>::advance(o.cb[l], x, b0, b1);
+            }
+        }
+    }
+    __device__ __forceinline__ int last_start(int l0) const {
+        int s = -1;
+        if (la >= l0 && la < kNoDegree) s = la;
+        if (lb >= l0 && lb < kNoDegree) s = max(s, lb);
+        return s;
+    }
+    __device__ __forceinline__ void start(const Order& o, int p, int l, const double2* __restrict__ pstart) {
+        if (la == l) {
+            const double2 ps = pstart[o.ra + p];
+            a0 = ps.x;
+            a1 = ps.y;
+        }
+        if (lb == l) {
+            const double2 ps = pstart[o.rb + p];
+            b0 = ps.x;
+            b1 = ps.y;
+        }
+        // a start at l + 1 is already the second element of the pair at l
+        if (la == l + 1) a1 = pstart[o.ra + p].x;
+        if (lb == l + 1) b1 = pstart[o.rb + p].x;
+    }
+    struct Coef {
+        double2 a, b;
+    };
+    static __device__ __forceinline__ Coef load(const Order& o, int l) { return {o.ca[l], o.cb[l]}; }
+    __device__ __forceinline__ void value(const VecFac<double>& f, int m, double& p0, double& p1) const {
+        p0 = fma(f.c1, m ? a0 : -b0, -(f.c2 * b0));  // Pbar^{-1} = -Pbar^1
+        p1 = fma(f.c3, a1, f.c4 * b1);
+    }
+    __device__ __forceinline__ void advance(const Coef& c) {
+        DirRec<double>::advance(c.a, x, a0, a1);
+        DirRec<double>::advance(c.b, x, b0, b1);
+    }
+};
+
+template <typename T, int CV, int R>
+constexpr int vec_min_ctas() {
+    return dir_min_ctas<T, 4 * CV, R>();
 }
 
 // ------------------------------------------------------------ analysis
-template <typename T>
-struct VFwdCfg {
-    static constexpr int LT = 32;   // degrees per tile
-    static constexpr int CT = 64;   // columns per CTA: 16 vector maps x (2 components x re, im)
-    static constexpr int RB = 128;  // rings generated per pass
-    static constexpr int KC = 16;   // rings per staged spectrum chunk
-};
-
-template <typename T>
-__host__ __device__ constexpr size_t vfwd_smem_bytes() {
-    using C = VFwdCfg<T>;
-    return (size_t)4 * C::LT * sizeof(double) + (size_t)C::RB * (C::LT + 1) * sizeof(double) +
-           (size_t)C::RB * 2 * C::LT * sizeof(T) + (size_t)2 * C::KC * 2 * C::CT * sizeof(T) + 64;
+template <typename T, int CV, int R>
+__host__ __device__ constexpr size_t vfwd_smem_bytes(int lch) {
+    return kDirWarps * (fwd_direct_xstride<T, 4 * CV, R>() * 2 * sizeof(T) + (size_t)lch * (8 * CV * sizeof(T) + sizeof(VecFac<T>)));
 }
 
-// Grid (Mv * ceil(Lv / LT), column tiles); CTA (m, jb) = blockIdx.x / nj, % nj.
-// spec: folded spectra [Mp][2][NP][C] of 2 * nvec scalar maps (column
-// 2 (2b + c) + {re, im}); alm: [nvec][2][Lv][Mv] complex.  use_nf = 0 leaves
-// out the 1/(l(l+1)) factor (the adjoint of the synthesis).
-template <typename T>
-__global__ void __launch_bounds__(256) k_vleg_fwd(const T* __restrict__ spec, int C, int nvec, T* __restrict__ alm,
-                                                  int Lv, int Mv, int Lp, int Mp, int Lpad, Geom geo,
-                                                  const RingPair* __restrict__ pairs, const int* __restrict__ lstart,
-                                                  const double2* __restrict__ pstart,
-                                                  const double2* __restrict__ coef, const double2* __restrict__ seeds,
-                                                  int csphase, int use_nf) {
-    using Cfg = VFwdCfg<T>;
-    constexpr int LT = Cfg::LT, CT = Cfg::CT, RB = Cfg::RB, KC = Cfg::KC;
+// CTA: orders m = 4 blockIdx.y + warp, degrees m + blockIdx.x lch .. + lch (lch a
+// multiple of 64: a block seed), vector maps CV blockIdx.z .. + CV; blockIdx.x =
+// nch clears the rows' m > l entries.  F: ring spectra of 2 nvec scalar maps;
+// alm: [nvec][2][Lv][Mv] complex.  adjoint: fold factors of the synthesis' adjoint.
+// use_nf = 0 leaves out the 1/(l(l+1)) factor (the adjoint of the synthesis).
+template <typename T, int CV, int R>
+__global__ void __launch_bounds__(32 * kDirWarps, vec_min_ctas<T, CV, R>())
+    k_vleg_fwd(const T* __restrict__ F, int64_t Ftot, int nvec, T* __restrict__ alm, int Lv, int Mv, int Lp, Geom geo,
+               const RingLite* __restrict__ rings, const double* __restrict__ z, const int* __restrict__ lstart,
+               const double2* __restrict__ pstart, const typename DirRec<T>::Coef* __restrict__ coef,
+               const double2* __restrict__ norm, int Lpad, const double2* __restrict__ seeds, int lch, int nch,
+               int csphase, int adjoint, int use_nf) {
+    constexpr int NC = 2 * CV;                             // complex columns
+    constexpr int NV = kSumVals<T>, G = NV / (8 * CV);     // degrees per transposed sum
+    static_assert(G >= 1 && (G == 1 || G % 2 == 0), "a group starts at an even l - m, or is one degree");
+    constexpr int W = kDirWarps;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int NP = geo.NP;
-    const int nj = (Lv + LT - 1) / LT;
-    const int m = blockIdx.x / nj, jb = blockIdx.x % nj;
-    const int l0 = m + jb * LT;
-    const int c0 = blockIdx.y * CT;
-    const int tid = threadIdx.x;
-    double* cf = (double*)smem_raw;              // [4][LT]
-    double* Pa = cf + 4 * LT;                    // [RB][LT+1] Pbar^{m-1}
-    T* Dt = (T*)(Pa + RB * (LT + 1));            // [RB][2][LT]
-    T* Xs = Dt + RB * 2 * LT;                    // [2][KC][2][CT]
-    const int vb0 = c0 / 4;
-
-    // the l < m triangle (and whole orders m >= Lv) are zero
-    if (jb == 0) {
-        const int lz = min(m, Lv);
-        for (int i = tid; i < lz * (CT / 4) * 2; i += blockDim.x) {
-            const int comp = i & 1, vb = vb0 + (i >> 1) % (CT / 4), l = (i >> 1) / (CT / 4);
-            if (vb < nvec && HPX_INB(2 * ((((int64_t)vb * 2 + comp) * Lv + l) * Mv + m) + 1, kExtAlm, 17))
-                *(cplx<T>*)(alm + 2 * ((((int64_t)vb * 2 + comp) * Lv + l) * Mv + m)) = {(T)0, (T)0};
-        }
+    const int b0 = blockIdx.z * CV;
+    if ((int)blockIdx.x == nch) {
+        for (int l = blockIdx.y; l < Lv; l += gridDim.y)
+            for (int cc = 0; cc < NC; ++cc) {
+                const int64_t row = (int64_t)(2 * b0 + cc) * Lv + l;
+                if (2 * b0 + cc >= 2 * nvec) break;
+                for (int m = l + 1 + threadIdx.x; m < Mv; m += blockDim.x)
+                    if (HPX_INB(2 * (row * Mv + m) + 1, kExtAlm, 17)) ((cplx<T>*)alm)[row * Mv + m] = {(T)0, (T)0};
+            }
+        return;
     }
-    if (m >= Lv || l0 >= Lv) return;
-    if (tid < LT) {
-        double c1, c2, c3, c4;
-        vec_coefs(l0 + tid, m, c1, c2, c3, c4);
-        cf[tid] = c1;
-        cf[LT + tid] = c2;
-        cf[2 * LT + tid] = c3;
-        cf[3 * LT + tid] = c4;
-    }
-    const int t0 = geo.first_ring(m);
-    const int K = NP - t0;
-    const int nbk = seed_blocks(Lp);
+    constexpr size_t XS = fwd_direct_xstride<T, 4 * CV, R>();
+    VecFac<T>* fac = (VecFac<T>*)smem_raw + (size_t)warp * lch;       // [W][lch]
+    cplx<T>* Xs = (cplx<T>*)((VecFac<T>*)smem_raw + (size_t)W * lch);  // [W][XS]: [north, south][column][32 R rings]
+    T* acc = (T*)(Xs + W * XS) + (size_t)warp * lch * 8 * CV;
+    const int m0 = blockIdx.y * W, m = m0 + warp;
+    const int i0 = blockIdx.x * lch, l0 = m + i0;
+    if (m0 + i0 >= Lv) return;
+    const bool active = m < Mv && l0 < Lv;
+    const int n = active ? min(lch, Lv - l0) : 0;
+    const int ng = (n + G - 1) / G;
+    for (int i = lane; i < ng * NV; i += 32) acc[i] = (T)0;
+    const int t0 = active ? geo.first_ring(m) : NP;
+    const int64_t mo = (int64_t)min(m, Mv - 1);
+    const double2* nm = norm + mo * Lpad;
+    const auto ord = VecGen<T>::order((int)mo, Mv + 1, Lp, Lpad, NP, coef, norm);
+    for (int i = lane; i < ng * G; i += 32) fac[i] = VecFac<T>::make(l0 + i, m, nm, Lv);
 
-    const int bl = tid & 15;   // vector map within the tile
-    const int dg = tid >> 4;   // degrees l0 + 2 dg, + 1
-    T A[2][4], B[2][4];
+    auto stage = [&](int pb) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+        for (int kk = 0; kk < R; ++kk) {
+            const int j = threadIdx.x & (W - 1), k = kk * 32 + threadIdx.x / W, p = pb + k, mj = m0 + j;
+            cplx<T>* xd = Xs + j * XS + k;
+            RingLite rl{};
+            if (p < NP) rl = rings[p];
+            const bool ok = mj < rl.mt && mj < Mv;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) A[i][k] = B[i][k] = (T)0;
-
-    auto stage = [&](int buf, int rbase, int nr) {
-        T* dst = Xs + buf * (KC * 2 * CT);
-        constexpr int VPR = CT * sizeof(T) / 16;
-        for (int i = tid; i < KC * 2 * VPR; i += blockDim.x) {
-            const int v = i % VPR, row = i / VPR;
-            const int q = row >> 1, pr = row & 1;
-            const int c = c0 + v * (16 / (int)sizeof(T));
-            const bool ok = q < nr && c < C;
-            const T* src = spec + (((int64_t)m * 2 + pr) * NP + t0 + (ok ? rbase + q : 0)) * C + (ok ? c : 0);
-            cp_async16(dst + row * CT + v * (16 / sizeof(T)), src, ok);
+            for (int cc = 0; cc < NC; ++cc) {
+                const int64_t fb = (int64_t)(2 * b0 + cc) * Ftot + mj;
+                const bool in = ok && 2 * b0 + cc < 2 * nvec;
+                if (in && HPX_INB(2 * (fb + rl.foff_n) + 1, kExtF, 25))
+                    cp_async_cplx(xd + cc * 32 * R, (const cplx<T>*)F + fb + rl.foff_n);
+                else
+                    xd[cc * 32 * R] = {(T)0, (T)0};
+                if (in && rl.foff_s >= 0 && HPX_INB(2 * (fb + rl.foff_s) + 1, kExtF, 25))
+                    cp_async_cplx(xd + (NC + cc) * 32 * R, (const cplx<T>*)F + fb + rl.foff_s);
+                else
+                    xd[(NC + cc) * 32 * R] = {(T)0, (T)0};
+            }
         }
         cp_async_commit();
     };
-
-    for (int rb = 0; rb < K; rb += RB) {
-        __syncthreads();  // coefficient factors ready / previous pass done with Pa, Dt
-        if (tid < RB) {
-            const int r = rb + tid;
-            double* pa = Pa + tid * (LT + 1);
-            T* d0 = Dt + tid * 2 * LT;
-            T* d1 = d0 + LT;
-            if (r < K) {
-                const int p = t0 + r;
-                const double x = pairs[p].z;
-                // order m+1 from its degree-block seed at or below l0 (values below m+1 are zero)
-                const int ob = m + 1;
-                const int jbb = l0 > ob ? (l0 - ob) / kSeedBlock : 0;
-                // order m-1 likewise (m = 0 uses Pbar^{-1} = -Pbar^1)
-                if (m >= 1) {
-                    const int oa = m - 1;
-                    const int jba = (l0 - oa) / kSeedBlock;
-                    const int64_t mia = (int64_t)oa * NP + p;
-                    const int ls = lstart[mia];
-                    const double2 ps = pstart[mia];
-                    const double2 sd = seeds[((int64_t)oa * nbk + jba) * NP + p];
-                    const double2* ca = coef + (int64_t)oa * Lpad;
-                    const int lsb = oa + jba * kSeedBlock;
-                    double q1 = 0.0, q2 = 0.0;
-                    for (int l = lsb; l <= l0 + LT; ++l) {
-                        double v;
-                        if (l == lsb && ls <= lsb) v = sd.x;
-                        else if (l == lsb + 1 && ls <= lsb) v = sd.y;
-                        else {
-                            const double2 ab = (l >= oa + 2 && l < Lp) ? ca[l] : make_double2(0.0, 0.0);
-                            v = l < Lp ? leg_step(l, ls, ps, ab.x, ab.y, x, q1, q2) : 0.0;
-                        }
-                        q2 = q1;
-                        q1 = v;
-                        if (l >= l0) pa[l - l0] = v;
-                    }
+    const int pfirst = geo.first_ring(m0);
+    if (pfirst < NP) stage(pfirst);
+    for (int pb = pfirst; pb < NP; pb += 32 * R) {
+        VecGen<T> gen[R];
+        int lmin = kNoDegree, lmax = -1;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int p = pb + 32 * r + lane;
+            gen[r].clear();
+            if (p >= t0 && p < NP) {
+                const int s = gen[r].init(ord, p, z[p], l0, l0 + n, lstart);
+                if (s < l0 + n) {
+                    gen[r].seed(ord, p, NP, l0, seeds, pstart);
+                    lmin = min(lmin, s);
+                    lmax = max(lmax, gen[r].last_start(l0));
                 }
-                const int64_t mib = (int64_t)ob * NP + p;
-                const int ls = ob < Mp ? lstart[mib] : Lp;
-                const double2 ps = ob < Mp ? pstart[mib] : make_double2(0.0, 0.0);
-                const int lsb = ob + jbb * kSeedBlock;
-                const double2 sd = (ob < Mp && lsb < Lp) ? seeds[((int64_t)ob * nbk + jbb) * NP + p] : make_double2(0.0, 0.0);
-                const double2* cb = coef + (int64_t)(ob < Mp ? ob : 0) * Lpad;
-                double q1 = 0.0, q2 = 0.0, prev = 0.0;
-                const int lstart_b = min(lsb, l0);
-                for (int l = lstart_b; l <= l0 + LT; ++l) {
-                    double v = 0.0;
-                    if (l >= ob && ob < Mp && l < Lp) {
-                        if (l == lsb && ls <= lsb) v = sd.x;
-                        else if (l == lsb + 1 && ls <= lsb) v = sd.y;
-                        else {
-                            const double2 ab = l >= ob + 2 ? cb[l] : make_double2(0.0, 0.0);
-                            v = leg_step(l, ls, ps, ab.x, ab.y, x, q1, q2);
-                        }
-                    }
-                    q2 = q1;
-                    q1 = v;
-                    if (l >= l0) {
-                        const int i = l - l0;
-                        const double pm = m >= 1 ? pa[i] : -v;  // Pbar_l^{m-1}
-                        if (i < LT) d0[i] = (T)((l >= m && l < Lv) ? cf[i] * pm - cf[LT + i] * v : 0.0);
-                        if (i > 0) {
-                            // D1 at degree l - 1 uses Pbar_l^{m-1} and Pbar_l^{m+1}
-                            const int ld = l - 1;
-                            d1[i - 1] = (T)((m >= 1 && ld >= m && ld < Lv) ? cf[2 * LT + i - 1] * pm + cf[3 * LT + i - 1] * v
-                                                                             : 0.0);
-                        }
-                    }
-                    prev = v;
-                }
-                (void)prev;
-            } else {
-                for (int i = 0; i < LT; ++i) d0[i] = d1[i] = (T)0;
             }
         }
-        const int rend = min(RB, K - rb);
-        const int nch = (rend + KC - 1) / KC;
-        stage(0, rb, min(KC, rend));
+        lmin = __reduce_min_sync(0xffffffffu, lmin);
+        lmax = __reduce_max_sync(0xffffffffu, lmax);
+        cp_async_wait<0>();
         __syncthreads();
-        for (int ch = 0; ch < nch; ++ch) {
-            if (ch + 1 < nch) {
-                stage((ch + 1) & 1, rb + (ch + 1) * KC, min(KC, rend - (ch + 1) * KC));
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
+        Pair<T> S[R][NC], D[R][NC];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int p = min(pb + 32 * r + lane, NP - 1);
+            const RingLite& rl = rings[p];
+            const bool south = rl.foff_s >= 0;
+            const double w0 = adjoint ? ((m == 0 || m == rl.h) ? 1.0 : 2.0) : rl.w;
+            const T w = (T)(VecGen<T>::kScaled ? w0 * rl.rs : w0);  // quadrature weight (/ sin(theta))
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) {
+                const cplx<T>* xs = Xs + warp * XS + 32 * r + lane;
+                const cplx<T> a = xs[cc * 32 * R], c = xs[(NC + cc) * 32 * R];
+                const cplx<T> sv = cscale(cadd(a, c), w), dv = cscale(csub(a, c), south ? w : (T)0);
+                S[r][cc] = Pair<T>::make(sv.re, sv.im);
+                D[r][cc] = Pair<T>::make(dv.re, dv.im);
             }
-            __syncthreads();
-            const T* xb = Xs + (ch & 1) * (KC * 2 * CT);
-            const int qn = min(KC, rend - ch * KC);
-            for (int q = 0; q < qn; ++q) {
-                const T* drow = Dt + (ch * KC + q) * 2 * LT;
+        }
+        __syncthreads();
+        if (pb + 32 * R < NP) stage(pb + 32 * R);
+        if (lmin == kNoDegree) continue;
+        // one group; ODD: its first degree has l - m odd (groups of one degree)
+        auto group = [&](int g, auto starts, auto odd) {
+            const int lg = l0 + g * G;
+            Pair<T> v[G][2][NC];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int li = 2 * dg + i;
-                    const int par0 = (li + 1) & 1;  // l - m = jb*LT + li, LT even
-                    const T d0 = drow[li], d1 = drow[LT + li];
-                    const T* x0 = xb + (q * 2 + par0) * CT + 4 * bl;
-                    const T* x1 = xb + (q * 2 + (par0 ^ 1)) * CT + 4 * bl;
+            for (int i = 0; i < G; ++i)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        A[i][k] = fma(d0, x0[k], A[i][k]);
-                        B[i][k] = fma(d1, x1[k], B[i][k]);
+                for (int cc = 0; cc < NC; ++cc) v[i][0][cc] = v[i][1][cc] = Pair<T>::zero();
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                const auto ab = VecGen<T>::load(ord, lg + i);
+                const VecFac<T> fl = fac[g * G + i];
+                const bool od = ((i & 1) != 0) != decltype(odd)::value;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if constexpr (decltype(starts)::value) gen[r].start(ord, pb + 32 * r + lane, lg + i, pstart);
+                    T p0, p1;
+                    gen[r].value(fl, m, p0, p1);
+                    const Pair<T> pp0 = Pair<T>::make(p0, p0), pp1 = Pair<T>::make(p1, p1);
+#pragma unroll
+                    for (int cc = 0; cc < NC; ++cc) {
+                        v[i][0][cc].fma(pp0, od ? S[r][cc] : D[r][cc]);
+                        v[i][1][cc].fma(pp1, od ? D[r][cc] : S[r][cc]);
                     }
+                    gen[r].advance(ab);
                 }
             }
-            __syncthreads();
-        }
-    }
-    // S = nf (A0 - i B1), T = nf (-A1 - i B0); A0 = (A[0], A[1]), A1 = (A[2], A[3]), likewise B
-    const int vb = vb0 + bl;
-    if (vb >= nvec) return;
+            T f[NV];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int l = l0 + 2 * dg + i;
-        if (l >= Lv) continue;
-        T nf = (l == 0 || !use_nf) ? (T)1 : (T)(1.0 / ((double)l * (double)(l + 1)));
-        if (csphase && (m & 1)) nf = -nf;
-        if (!HPX_INB(2 * ((((int64_t)vb * 2 + 1) * Lv + l) * Mv + m) + 1, kExtAlm, 18)) continue;
-        const cplx<T> S = {nf * (A[i][0] + B[i][3]), nf * (A[i][1] - B[i][2])};
-        const cplx<T> Tt = {nf * (B[i][1] - A[i][2]), -nf * (A[i][3] + B[i][0])};
-        *(cplx<T>*)(alm + 2 * ((((int64_t)vb * 2 + 0) * Lv + l) * Mv + m)) = S;
-        *(cplx<T>*)(alm + 2 * ((((int64_t)vb * 2 + 1) * Lv + l) * Mv + m)) = Tt;
+            for (int i = 0; i < G; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int cc = 0; cc < NC; ++cc) {
+                        const auto q = v[i][h][cc].get();
+                        f[(i * 2 + h) * 2 * NC + 2 * cc] = q.x;
+                        f[(i * 2 + h) * 2 * NC + 2 * cc + 1] = q.y;
+                    }
+            const T sum = transpose_sum(f, lane);
+            if (lane < NV) acc[g * NV + lane] += sum;
+        };
+        int g = max(0, lmin - l0) / G;
+        const int gs = lmax < 0 ? g : min(ng, (lmax - l0) / G + 1);
+        auto run = [&](int gend, auto starts) {
+            if constexpr (G == 1) {
+                // l0 - m is a multiple of 64: group g has parity g & 1
+                if (g < gend && (g & 1)) {
+                    group(g, starts, DirYes{});
+                    ++g;
+                }
+#pragma unroll 1
+                for (; g + 1 < gend; g += 2) {
+                    group(g, starts, DirNo{});
+                    group(g + 1, starts, DirYes{});
+                }
+                if (g < gend) {
+                    group(g, starts, DirNo{});
+                    ++g;
+                }
+            } else {
+#pragma unroll 1
+                for (; g < gend; ++g) group(g, starts, DirNo{});
+            }
+        };
+        run(gs, DirYes{});
+        run(ng, DirNo{});
+    }
+    __syncwarp();
+    // S = nf (A0 - i B1), T = nf (-A1 - i B0); A: D0 sums, B: D1 sums of the two components
+    for (int i = lane; i < n; i += 32) {
+        const int l = l0 + i;
+        double c = sizeof(T) == 4 ? nm[l].x : 1.0;
+        if (use_nf && l > 0) c *= 1.0 / ((double)l * (double)(l + 1));
+        if (csphase && (m & 1)) c = -c;
+        const double cb = VecGen<T>::kScaled ? c * m : c;
+#pragma unroll
+        for (int vb = 0; vb < CV; ++vb) {
+            if (b0 + vb >= nvec) break;
+            const cplx<T>* a = (const cplx<T>*)(acc + (size_t)i * 8 * CV) + 2 * vb;
+            const cplx<T>* b = a + NC;
+            const int64_t o = ((int64_t)(b0 + vb) * 2 * Lv + l) * Mv + m;
+            if (!HPX_INB(2 * (o + (int64_t)Lv * Mv) + 1, kExtAlm, 18)) continue;
+            ((cplx<T>*)alm)[o] = {(T)(c * a[0].re + cb * b[1].im), (T)(c * a[0].im - cb * b[1].re)};
+            ((cplx<T>*)alm)[o + (int64_t)Lv * Mv] = {(T)(cb * b[0].im - c * a[1].re), (T)(-(c * a[1].im + cb * b[0].re))};
+        }
     }
 }
 
 // ------------------------------------------------------------ synthesis
-template <typename T>
-struct VInvCfg {
-    static constexpr int RBI = 64;  // rings per CTA
-    static constexpr int CT = 64;   // columns per CTA (16 vector maps)
-    static constexpr int LC = 32;   // degrees per staged chunk
-};
-
-template <typename T>
+template <typename T, int CV, int R>
 __host__ __device__ constexpr size_t vinv_smem_bytes() {
-    using C = VInvCfg<T>;
-    return (size_t)4 * C::LC * sizeof(double) + (size_t)2 * C::LC * C::RBI * sizeof(T) +
-           (size_t)C::LC * C::CT * sizeof(T) + 64;
+    const size_t raw = (size_t)2 * kDirWarps * kDirChunk * 2 * CV * 2 * sizeof(T);
+    const size_t rows = (size_t)kDirWarps * kDirChunk * (8 * CV * sizeof(T) + sizeof(VecFac<T>));
+    const size_t f = (size_t)2 * kDirWarps * 32 * R * 4 * CV * sizeof(T);
+    return raw + rows > f ? raw + rows : f;
 }
 
-// Grid (Mp * ceil(NP / RBI), column tiles); CTA (m, ring block) = blockIdx.x / nr, % nr.
-// Writes E/O spectra spec[m][0|1][p][C] of the 2 nvec scalar maps for every
-// m < Mp and ring p >= first_ring(m) (zeros for orders the coefficients do not carry).
-// use_nf = 1 first scales the coefficients by 1/(l(l+1)) (the adjoint of the analysis).
-template <typename T>
-__global__ void __launch_bounds__(256) k_vleg_inv(const T* __restrict__ alm, int nvec, T* __restrict__ spec, int C,
-                                                  int Lv, int Mv, int Lp, int Mp, int Lpad, Geom geo,
-                                                  const RingPair* __restrict__ pairs, const int* __restrict__ lstart,
-                                                  const double2* __restrict__ pstart,
-                                                  const double2* __restrict__ coef, int csphase, int use_nf) {
-    using Cfg = VInvCfg<T>;
-    constexpr int RBI = Cfg::RBI, CT = Cfg::CT, LC = Cfg::LC;
+// CTA: orders m = 4 blockIdx.y + warp < Mp, rings 32 R blockIdx.x .. + 32 R, vector
+// maps CV blockIdx.z .. + CV (as k_leg_inv_direct).  Orders the coefficients do not
+// carry get zero spectra.  use_nf = 1 first scales the coefficients by 1/(l(l+1))
+// (the adjoint of the analysis, whose fold factors `adjoint` selects).
+template <typename T, int CV, int R>
+__global__ void __launch_bounds__(32 * kDirWarps, vec_min_ctas<T, CV, R>())
+    k_vleg_inv(const T* __restrict__ alm, int nvec, T* __restrict__ F, int64_t Ftot, int Lv, int Mv, int Lp, int Mp,
+               Geom geo, const RingLite* __restrict__ rings, const double* __restrict__ z,
+               const int* __restrict__ lstart, const double2* __restrict__ pstart,
+               const typename DirRec<T>::Coef* __restrict__ coef, const double2* __restrict__ norm, int Lpad,
+               const double2* __restrict__ seeds, int csphase, int adjoint, int use_nf) {
+    constexpr int NC = 2 * CV, W = kDirWarps, LC = kDirChunk;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_first;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    VecFac<T>* fac = (VecFac<T>*)smem_raw + warp * LC;                      // [W][LC]
+    cplx<T>* raw = (cplx<T>*)((VecFac<T>*)smem_raw + W * LC);               // [2][W][LC][NC]: (S, T) per map
+    T* rows = (T*)(raw + 2 * W * LC * NC) + (size_t)warp * LC * 8 * CV;     // [W][LC][A0, A1][2 NC]
     const int NP = geo.NP;
-    const int nr = (NP + RBI - 1) / RBI;
-    const int m = blockIdx.x / nr, rb = (blockIdx.x % nr) * RBI;
-    const int c0 = blockIdx.y * CT;
-    const int tid = threadIdx.x;
-    const int t0 = geo.first_ring(m);
-    const int K = NP - t0;
-    if (rb >= K) return;
-    double* cf = (double*)smem_raw;       // [4][LC]
-    T* D0 = (T*)(cf + 4 * LC);            // [LC][RBI]
-    T* D1 = D0 + LC * RBI;                // [LC][RBI]
-    T* As = D1 + LC * RBI;                // [LC][CT]: per vector map S re, S im, T re, T im
+    const int m0 = blockIdx.y * W, m = m0 + warp;
+    const int pb = blockIdx.x * 32 * R;
+    const int b0 = blockIdx.z * CV;
+    if (pb + 32 * R <= geo.first_ring(m0)) return;
+    const int mend = min(Mv, Lv);  // orders with coefficients
+    const int t0 = m < mend ? geo.first_ring(m) : NP;
+    const int64_t mo = min(m, Mp - 1);
+    const double2* nm = norm + mo * Lpad;
+    const auto ord = VecGen<T>::order((int)mo, Mp, Lp, Lpad, NP, coef, norm);
 
-    const int tx = tid & 15, ty = tid >> 4;
-    const int rrow = ty * 4;
-    T E[4][4], O[4][4];
+    VecGen<T> gen[R];
+    int lmin = kNoDegree, lmax = -1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) E[i][k] = O[i][k] = (T)0;
-
-    if (m < Mv && m < Lv) {
-        // generator threads: one ring each, running orders m-1 and m+1 one degree ahead
-        const int rg = rb + tid;
-        const bool gen = tid < RBI && rg < K;
-        LegRun ra, rbn;
-        double cur_a = 0.0, nxt_a = 0.0, cur_b = 0.0, nxt_b = 0.0;
-        const double2* ca = coef + (int64_t)(m >= 1 ? m - 1 : 0) * Lpad;
-        const double2* cb = coef + (int64_t)(m + 1) * Lpad;
-        if (gen) {
-            const int p = t0 + rg;
-            const double x = pairs[p].z;
-            if (m >= 1) ra.init(m - 1, Mp, Mp, (int64_t)(m - 1) * NP + p, lstart, pstart, x);
-            rbn.init(m + 1, Mp, Mp, (int64_t)(m + 1) * NP + p, lstart, pstart, x);
-            // degree m: Pbar_m^{m-1} needs the run from m-1; Pbar_m^{m+1} = 0
-            if (m >= 1) {
-                ra.next(ca, Lp);           // degree m-1
-                cur_a = ra.next(ca, Lp);   // degree m
-                nxt_a = ra.next(ca, Lp);   // degree m+1
-            }
-            cur_b = 0.0;
-            nxt_b = rbn.next(cb, Lp);      // degree m+1
-        }
-        for (int l0 = m; l0 < Lv; l0 += LC) {
-            __syncthreads();  // previous chunk consumed
-            if (tid < LC) {
-                double c1, c2, c3, c4;
-                vec_coefs(l0 + tid, m, c1, c2, c3, c4);
-                cf[tid] = c1;
-                cf[LC + tid] = c2;
-                cf[2 * LC + tid] = c3;
-                cf[3 * LC + tid] = c4;
-            }
-            for (int i = tid; i < LC * CT; i += blockDim.x) {
-                const int c = i % CT, li = i / CT, l = l0 + li;
-                const int vb = (c0 + c) >> 2, k = c & 3;  // k: S re, S im, T re, T im
-                T v = (T)0;
-                if (l < Lv && vb < nvec) v = alm[2 * ((((int64_t)vb * 2 + (k >> 1)) * Lv + l) * Mv + m) + (k & 1)];
-                if (use_nf && l > 0) v = (T)((double)v / ((double)l * (double)(l + 1)));
-                As[li * CT + c] = v;
-            }
-            __syncthreads();
-            if (tid < RBI) {
-                for (int i = 0; i < LC; ++i) {
-                    const int l = l0 + i;
-                    double d0 = 0.0, d1 = 0.0;
-                    if (gen && l < Lv) {
-                        const double pa = m >= 1 ? cur_a : -cur_b;
-                        d0 = cf[i] * pa - cf[LC + i] * cur_b;
-                        d1 = m >= 1 ? cf[2 * LC + i] * nxt_a + cf[3 * LC + i] * nxt_b : 0.0;
-                        cur_a = nxt_a;
-                        cur_b = nxt_b;
-                        if (m >= 1) nxt_a = ra.next(ca, Lp);
-                        nxt_b = rbn.next(cb, Lp);
-                    }
-                    if (csphase && (m & 1)) {
-                        d0 = -d0;
-                        d1 = -d1;
-                    }
-                    D0[i * RBI + tid] = (T)d0;
-                    D1[i * RBI + tid] = (T)d1;
-                }
-            }
-            __syncthreads();
-            for (int li = 0; li < LC; ++li) {
-                const int l = l0 + li;
-                const bool even = ((l + m) & 1) == 0;
-                const T* ar = As + li * CT + 4 * tx;
-                const T sr = ar[0], si = ar[1], tr = ar[2], ti = ar[3];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const T d0 = D0[li * RBI + rrow + i], d1 = D1[li * RBI + rrow + i];
-                    // D0 part (south sign -(-1)^{l+m}) and D1 part (south sign (-1)^{l+m})
-                    const T p0[4] = {d0 * sr, d0 * si, -d0 * tr, -d0 * ti};
-                    const T p1[4] = {-d1 * ti, d1 * tr, -d1 * si, d1 * sr};
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        E[i][k] += even ? p1[k] : p0[k];
-                        O[i][k] += even ? p0[k] : p1[k];
-                    }
-                }
+    for (int r = 0; r < R; ++r) {
+        const int p = pb + 32 * r + lane;
+        gen[r].clear();
+        if (p >= t0 && p < NP) {
+            const int s = gen[r].init(ord, p, z[p], m, Lv, lstart);
+            if (s < Lv) {
+                gen[r].seed(ord, p, NP, m, seeds, pstart);
+                lmin = min(lmin, s);
+                lmax = max(lmax, gen[r].last_start(m));
             }
         }
     }
-    // write E/O for the rings of this CTA
+    lmin = __reduce_min_sync(0xffffffffu, lmin);
+    lmax = __reduce_max_sync(0xffffffffu, lmax);
+    if (threadIdx.x == 0) s_first = kNoDegree;
+    __syncthreads();
+    if (lane == 0 && lmin < kNoDegree) atomicMin(&s_first, lmin - m);
+    __syncthreads();
+    const int ibeg = s_first == kNoDegree ? Lv : s_first & ~(LC - 1);
+
+    auto stage = [&](int buf, int i0) {
+        cplx<T>* dst = raw + (size_t)buf * W * LC * NC;
+        const int j = threadIdx.x & (W - 1), mm = m0 + j;
+        const int64_t lm = (int64_t)Lv * Mv;
+        for (int k = threadIdx.x / W; k < LC + W - 1; k += 32) {
+            const int i = k - j, l = m0 + i0 + k;
+            if (i < 0 || i >= LC) continue;
+            cplx<T>* d = dst + (j * LC + i) * NC;
+            const bool ok = l < Lv && mm < Mv;
+            const int64_t o = (int64_t)2 * b0 * lm + (int64_t)l * Mv + mm;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = rb + rrow + i;
-        if (r >= K || c0 + 4 * tx >= C || !HPX_INB((((int64_t)m * 2 + 1) * NP + t0 + r) * C + c0 + 4 * tx + 3, kExtSpec, 19))
-            continue;
-        T* e = spec + (((int64_t)m * 2 + 0) * NP + t0 + r) * C + c0 + 4 * tx;
-        T* o = spec + (((int64_t)m * 2 + 1) * NP + t0 + r) * C + c0 + 4 * tx;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (c0 + 4 * tx + k < C) {
-                e[k] = E[i][k];
-                o[k] = O[i][k];
+            for (int cc = 0; cc < NC; ++cc) {
+                if (ok && 2 * b0 + cc < 2 * nvec && HPX_INB(2 * (o + cc * lm) + 1, kExtAlm, 26))
+                    cp_async_cplx(d + cc, (const cplx<T>*)alm + o + cc * lm);
+                else
+                    d[cc] = {(T)0, (T)0};
             }
+        }
+        cp_async_commit();
+    };
+
+    Pair<T> E[R][NC], O[R][NC];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) E[r][cc] = O[r][cc] = Pair<T>::zero();
+    constexpr int G = 4;  // degrees per unrolled group
+
+    int buf = 0;
+    if (m0 + ibeg < Lv) stage(0, ibeg);
+    for (int i0 = ibeg; m0 + i0 < Lv; i0 += LC, buf ^= 1) {
+        if (m0 + i0 + LC < Lv) {
+            stage(buf ^ 1, i0 + LC);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        const int lc = m + i0;
+        if (lc < Lv && lmin < lc + LC) {
+            // rows of degree lc + lane: A0 = c (S, -T), A1 = c m (i T, i S) as re, im pairs
+            const int l = lc + lane;
+            fac[lane] = VecFac<T>::make(l, m, nm, Lv);
+            double c = sizeof(T) == 4 && l < Lv ? nm[l].x : 1.0;
+            if (use_nf && l > 0) c *= 1.0 / ((double)l * (double)(l + 1));
+            if (csphase && (m & 1)) c = -c;
+            const double cb = VecGen<T>::kScaled ? c * m : c;
+            const cplx<T>* sr = raw + ((size_t)(buf * W + warp) * LC + lane) * NC;
+            cplx<T>* row = (cplx<T>*)(rows + lane * 8 * CV);
+#pragma unroll
+            for (int vb = 0; vb < CV; ++vb) {
+                const cplx<T> Sv = sr[2 * vb], Tv = sr[2 * vb + 1];
+                row[2 * vb] = {(T)(c * Sv.re), (T)(c * Sv.im)};
+                row[2 * vb + 1] = {(T)(-c * Tv.re), (T)(-c * Tv.im)};
+                row[NC + 2 * vb] = {(T)(-cb * Tv.im), (T)(cb * Tv.re)};
+                row[NC + 2 * vb + 1] = {(T)(-cb * Sv.im), (T)(cb * Sv.re)};
+            }
+            __syncwarp();
+            auto group = [&](int k, auto starts) {
+                const int lg = lc + k;
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    const auto ab = VecGen<T>::load(ord, lg + i);
+                    const VecFac<T> fl = fac[k + i];
+                    Pair<T> a0[NC], a1[NC];
+                    load_pairs<NC>(a0, rows + (k + i) * 8 * CV);
+                    load_pairs<NC>(a1, rows + (k + i) * 8 * CV + 2 * NC);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        if constexpr (decltype(starts)::value) gen[r].start(ord, pb + 32 * r + lane, lg + i, pstart);
+                        T p0, p1;
+                        gen[r].value(fl, m, p0, p1);
+                        const Pair<T> pp0 = Pair<T>::make(p0, p0), pp1 = Pair<T>::make(p1, p1);
+#pragma unroll
+                        for (int cc = 0; cc < NC; ++cc) {
+                            ((i & 1) ? E[r][cc] : O[r][cc]).fma(pp0, a0[cc]);
+                            ((i & 1) ? O[r][cc] : E[r][cc]).fma(pp1, a1[cc]);
+                        }
+                        gen[r].advance(ab);
+                    }
+                }
+            };
+            int k = max(0, lmin - lc) & ~(G - 1);
+            const int kend = min(LC, Lv - lc);
+            const int ks = min(kend, max(0, lmax - lc + 1));
+#pragma unroll 1
+            for (; k < ks; k += G) group(k, DirYes{});
+#pragma unroll 1
+            for (; k < kend; k += G) group(k, DirNo{});
+        }
+        __syncthreads();
+    }
+    cplx<T>* Fo = (cplx<T>*)smem_raw;  // [E + O, E - O][column][ring][order]
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) {
+            const auto e = E[r][cc].get(), o = O[r][cc].get();
+            const int k = 32 * r + lane;
+            Fo[(cc * 32 * R + k) * W + (warp ^ (k & (W - 1)))] = {e.x + o.x, e.y + o.y};
+            Fo[((NC + cc) * 32 * R + k) * W + (warp ^ (k & (W - 1)))] = {e.x - o.x, e.y - o.y};
+        }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < R; ++kk) {
+        const int j = threadIdx.x & (W - 1), k = kk * 32 + threadIdx.x / W, p = pb + k, mj = m0 + j;
+        if (p >= NP) continue;
+        const RingLite rl = rings[p];
+        if (mj >= rl.mt) continue;
+        double s0 = 1.0;
+        if (adjoint) s0 = (mj == 0 || mj == rl.h) ? rl.w : 0.5 * rl.w;
+        const T sc = (T)(VecGen<T>::kScaled ? s0 * rl.rs : s0);
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) {
+            if (2 * b0 + cc >= 2 * nvec) break;
+            const int64_t fb = (int64_t)(2 * b0 + cc) * Ftot + mj;
+            const int jj = j ^ (k & (W - 1));
+            if (HPX_INB(2 * (fb + rl.foff_n) + 1, kExtF, 19))
+                ((cplx<T>*)F)[fb + rl.foff_n] = cscale(Fo[(cc * 32 * R + k) * W + jj], sc);
+            if (rl.foff_s >= 0 && HPX_INB(2 * (fb + rl.foff_s) + 1, kExtF, 19))
+                ((cplx<T>*)F)[fb + rl.foff_s] = cscale(Fo[((NC + cc) * 32 * R + k) * W + jj], sc);
         }
     }
 }
