@@ -72,32 +72,82 @@ __device__ __forceinline__ cplx<T>* ring_bluestein_tables(cplx<T>* smem, const R
     return csm + rp.h + ((half + rp.h) & 1);  // the buffers start 16-byte aligned
 }
 
-// The ring kernels come in three instantiations launched over three ring
-// lists: power-of-two rings (KIND 0, 3 CTAs per SM for float), Bluestein rings
-// of length 2^logP (KIND 1, 2 CTAs per SM with 128 registers and the ring's
-// tables in shared memory) and of length 3 * 2^logP (KIND 2, 3072 points: one
-// group of 192 threads, 2 CTAs per SM).  CTA (blockIdx.x, blockIdx.y) runs ring
-// rings[blockIdx.x] for its group of maps.
+// The ring kernels come in three kinds over three lists of ring pairs:
+// power-of-two rings (KIND 0, 3 CTAs per SM for float), Bluestein rings of length
+// 2^logP (KIND 1, 2 CTAs per SM with 128 registers and the ring's tables in shared
+// memory) and of length 3 * 2^logP (KIND 2, 3072 points: one group of 192
+// threads, 2 CTAs per SM).  CTA (x, y) runs pair rings[x] for its group of maps:
+// both its rings (BOTH) or, with many maps, the ring on side z.  North and south
+// share the pair's tables, so a CTA of one map already uses them twice: a call of
+// one map at nside 1024 went from 154 / 162 us (analysis / synthesis) to 115 /
+// 116 us, at nside 256 from 32 / 34 us to 22 / 23 us.
 template <typename T, int KIND>
 constexpr int ring_kernel_ctas() { return KIND ? 2 : ring_min_ctas<T>(); }
 template <int KIND>
 HPX_HD constexpr int ring_kernel_threads() { return KIND == 2 ? 192 : 256; }
 
-// One CTA per (ring t, group of maps): map[b][ring t] -> F[b][foff_t + m]
-template <typename T, int KIND>
-__global__ void __launch_bounds__(ring_kernel_threads<KIND>(), ring_kernel_ctas<T, KIND>())
-    k_ring_fwd(const T* __restrict__ map, int nmaps, int maps_per_cta, T* __restrict__ F, int64_t Ftot, Geom geo,
-               const RingPair* __restrict__ pairs, const int* __restrict__ rings, const cplx<T>* __restrict__ rtab,
-               int rslot, const cplx<T>* __restrict__ gtab, const cplx<T>* __restrict__ chirp,
-               unsigned* __restrict__ fmax) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int NP = geo.NP, R = geo.R;
-    const int t = rings[blockIdx.x];
-    const bool south = t >= NP;
-    const int pr = south ? R - 1 - t : t;
-    const RingPair rp = pairs[pr];
+// The rings of one pair and a group of maps as a sequence of transforms.  BOTH:
+// item q is the north or south ring of map q / 2; otherwise map q's ring on the
+// side z (0 north, 1 south), whose offsets then stay in registers (a run-time
+// side measured 3% slower at nside 1024, 64 maps).
+template <bool BOTH>
+struct RingItems {
+    int ns, z, q0, q1, shift_n, shift_s;
+    int64_t start_n, start_s, foff_n, foff_s;
+    __device__ __forceinline__ RingItems(const RingPair& rp, int side, int group, int maps_per_cta, int nmaps) {
+        ns = BOTH && rp.has_south ? 2 : 1;
+        z = side;
+        q0 = group * maps_per_cta * ns;
+        q1 = min((group + 1) * maps_per_cta, nmaps) * ns;
+        const bool s = !BOTH && side;
+        start_n = s ? rp.start_s : rp.start_n;
+        foff_n = s ? rp.foff_s : rp.foff_n;
+        shift_n = s ? rp.shift_s : rp.shift_n;
+        if (BOTH) {
+            start_s = rp.start_s;
+            foff_s = rp.foff_s;
+            shift_s = rp.shift_s;
+        }
+    }
+    __device__ __forceinline__ int map(int q) const { return BOTH && ns == 2 ? q >> 1 : q; }
+    __device__ __forceinline__ bool second(int q) const { return BOTH && ns == 2 && (q & 1); }
+    __device__ __forceinline__ int64_t start(int q) const { return second(q) ? start_s : start_n; }
+    __device__ __forceinline__ int64_t foff(int q) const { return second(q) ? foff_s : foff_n; }
+    __device__ __forceinline__ int shift(int q) const { return second(q) ? shift_s : shift_n; }
+};
+
+// Pair and side of this CTA.  One ring a CTA: the power-of-two rings from north to
+// south, as they lie in memory; the north and south rings of a Bluestein pair,
+// which share its tables in L2, side by side.
+template <int KIND, bool BOTH>
+__device__ __forceinline__ int2 ring_cta() {
+    const int x = blockIdx.x, n = gridDim.x >> 1;
+    if (BOTH) return make_int2(x, 0);
+    if (KIND == 0) return x < n ? make_int2(x, 0) : make_int2(2 * n - 1 - x, 1);
+    return make_int2(x >> 1, x & 1);
+}
+
+struct RingFwdArgs {
+    int nmaps, maps_per_cta;
+    int64_t Ftot;
+    Geom geo;
+    const RingPair* pairs;
+    const int* rings;
+    int rslot;
+    unsigned* fmax;
+};
+
+// map[b][ring] -> F[b][foff + m] for the pair args.rings[x] and map group y
+template <typename T, int KIND, bool BOTH>
+__device__ __forceinline__ void ring_fwd_cta(unsigned char* smem_raw, const RingFwdArgs& a, int x, int y, int z,
+                                             const T* __restrict__ map, T* __restrict__ F,
+                                             const cplx<T>* __restrict__ rtab, const cplx<T>* __restrict__ gtab,
+                                             const cplx<T>* __restrict__ chirp) {
+    const int pr = a.rings[x];
+    const RingPair rp = a.pairs[pr];
+    if (z && !rp.has_south) return;
     PhaseTab<T> E, tw;
-    cplx<T>* bufs = ring_tables<KIND>(smem_raw, rp, rtab + (size_t)pr * rslot, E, tw);
+    cplx<T>* bufs = ring_tables<KIND>(smem_raw, rp, rtab + (size_t)pr * a.rslot, E, tw);
     const cplx<T>* Gs = nullptr;
     const cplx<T>* cs = nullptr;
     if constexpr (KIND > 0) bufs = ring_bluestein_tables<KIND>(bufs, rp, gtab, chirp, Gs, cs);
@@ -107,51 +157,79 @@ __global__ void __launch_bounds__(ring_kernel_threads<KIND>(), ring_kernel_ctas<
     const int PL = padded_len(P);
     cplx<T>* buf = bufs + (size_t)g * 2 * PL;
     cplx<T>* buf2 = buf + PL;
-    const int64_t start = south ? rp.start_s : rp.start_n;
-    const int64_t foff = south ? rp.foff_s : rp.foff_n;
-    const int shift = south ? rp.shift_s : rp.shift_n;
-    const int64_t np = geo.npix;
-    const int b0 = blockIdx.y * maps_per_cta;
-    const int b1 = min(b0 + maps_per_cta, nmaps);
-    // (bounds-checked builds) the CTA's first and last maps' ring and spectrum
-    if (b1 > b0 && !(HPX_INB(b0 * np + start, kExtMap, 1) && HPX_INB((b1 - 1) * np + start + 2 * rp.h - 1, kExtMap, 1) &&
-                     HPX_INB(2 * ((int64_t)(b1 - 1) * Ftot + foff + rp.mt) - 1, kExtF, 2)))
-        return;
+    const int64_t np = a.geo.npix;
+    const RingItems<BOTH> it(rp, z, y, a.maps_per_cta, a.nmaps);
+    // (bounds-checked builds) the CTA's first and last rings and spectra
+    if (it.q1 > it.q0) {
+        const int b0 = it.map(it.q0), b1 = it.map(it.q1 - 1);
+        if (!(HPX_INB(b0 * np + it.start(it.q0), kExtMap, 1) &&
+              HPX_INB(b1 * np + it.start(it.q1 - 1) + 2 * rp.h - 1, kExtMap, 1) &&
+              HPX_INB(2 * ((int64_t)b1 * a.Ftot + it.foff(it.q1 - 1) + rp.mt) - 1, kExtF, 2)))
+            return;
+    }
+    auto ring = [&](int q) { return map + (int64_t)it.map(q) * np + it.start(q); };
     cplx<T>* cur = buf;
     cplx<T>* other = buf2;
-    if (b0 + g < b1) ring_load_async(cur, map + (int64_t)(b0 + g) * np + start, rp.h, lt, tpf);
-    for (int b = b0 + g; b < b1; b += S) {
+    if (it.q0 + g < it.q1) ring_load_async(cur, ring(it.q0 + g), rp.h, lt, tpf);
+    for (int q = it.q0 + g; q < it.q1; q += S) {
         auto load_next = [&](cplx<T>* dst) {
-            if (b + S < b1) ring_load_async(dst, map + (int64_t)(b + S) * np + start, rp.h, lt, tpf);
+            if (q + S < it.q1) ring_load_async(dst, ring(q + S), rp.h, lt, tpf);
         };
-        const T mx = ring_forward<KIND>(cur, other, shift, F + 2 * ((int64_t)b * Ftot + foff), rp, tw, Gs, cs, E, lt,
-                                        tpf, g, load_next);
-        if (fmax) {
+        const int b = it.map(q);
+        const T mx = ring_forward<KIND>(cur, other, it.shift(q), F + 2 * ((int64_t)b * a.Ftot + it.foff(q)), rp, tw, Gs,
+                                        cs, E, lt, tpf, g, load_next);
+        if (a.fmax) {
             // per-map max |F| (scale of the FP16 operands); a group is whole warps
             float v = (float)mx;
 #pragma unroll
             for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-            if ((threadIdx.x & 31) == 0 && v > 0.f) atomicMax(fmax + b, __float_as_uint(v));
+            if ((threadIdx.x & 31) == 0 && v > 0.f) atomicMax(a.fmax + b, __float_as_uint(v));
         }
     }
 }
 
-// One CTA per (ring t, group of maps): F[b][foff_t + m] -> map[b][ring t]
-// (ref != nullptr: write ref - synthesis)
-template <typename T, int KIND>
+template <typename T, int KIND, bool BOTH>
 __global__ void __launch_bounds__(ring_kernel_threads<KIND>(), ring_kernel_ctas<T, KIND>())
-    k_ring_inv(const T* __restrict__ F, int64_t Ftot, T* __restrict__ map, int nmaps, int maps_per_cta, Geom geo,
-               const RingPair* __restrict__ pairs, const int* __restrict__ rings, const cplx<T>* __restrict__ rtab,
-               int rslot, const cplx<T>* __restrict__ gtab, const cplx<T>* __restrict__ chirp,
-               const T* __restrict__ ref) {
+    k_ring_fwd(RingFwdArgs a, const T* __restrict__ map, T* __restrict__ F, const cplx<T>* __restrict__ rtab,
+               const cplx<T>* __restrict__ gtab, const cplx<T>* __restrict__ chirp) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int NP = geo.NP, R = geo.R;
-    const int t = rings[blockIdx.x];
-    const bool south = t >= NP;
-    const int pr = south ? R - 1 - t : t;
-    const RingPair rp = pairs[pr];
+    const int2 c = ring_cta<KIND, BOTH>();
+    ring_fwd_cta<T, KIND, BOTH>(smem_raw, a, c.x, blockIdx.y, c.y, map, F, rtab, gtab, chirp);
+}
+
+// Kinds 0 and 1 in one launch, for calls too small to fill the GPU: the Bluestein
+// pairs (the longer work) first, then the power-of-two ones.
+template <typename T>
+__global__ void __launch_bounds__(256, ring_kernel_ctas<T, 1>())
+    k_ring_fwd_any(RingFwdArgs a, int n_blue, int n_pow2, const T* __restrict__ map, T* __restrict__ F,
+                   const cplx<T>* __restrict__ rtab, const cplx<T>* __restrict__ gtab,
+                   const cplx<T>* __restrict__ chirp) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int x = blockIdx.x;
+    if (x < n_blue) ring_fwd_cta<T, 1, true>(smem_raw, a, n_pow2 + x, blockIdx.y, 0, map, F, rtab, gtab, chirp);
+    else ring_fwd_cta<T, 0, true>(smem_raw, a, x - n_blue, blockIdx.y, 0, map, F, rtab, gtab, chirp);
+}
+
+struct RingInvArgs {
+    int nmaps, maps_per_cta;
+    int64_t Ftot;
+    Geom geo;
+    const RingPair* pairs;
+    const int* rings;
+    int rslot;
+};
+
+// F[b][foff + m] -> map[b][ring] (ref != nullptr: write ref - synthesis)
+template <typename T, int KIND, bool BOTH>
+__device__ __forceinline__ void ring_inv_cta(unsigned char* smem_raw, const RingInvArgs& a, int x, int y, int z,
+                                             const T* __restrict__ F, T* __restrict__ map,
+                                             const cplx<T>* __restrict__ rtab, const cplx<T>* __restrict__ gtab,
+                                             const cplx<T>* __restrict__ chirp, const T* __restrict__ ref) {
+    const int pr = a.rings[x];
+    const RingPair rp = a.pairs[pr];
+    if (z && !rp.has_south) return;
     PhaseTab<T> E, tw;
-    cplx<T>* bufs = ring_tables<KIND>(smem_raw, rp, rtab + (size_t)pr * rslot, E, tw);
+    cplx<T>* bufs = ring_tables<KIND>(smem_raw, rp, rtab + (size_t)pr * a.rslot, E, tw);
     const cplx<T>* Gs = nullptr;
     const cplx<T>* cs = nullptr;
     if constexpr (KIND > 0) bufs = ring_bluestein_tables<KIND>(bufs, rp, gtab, chirp, Gs, cs);
@@ -161,26 +239,47 @@ __global__ void __launch_bounds__(ring_kernel_threads<KIND>(), ring_kernel_ctas<
     const int PL = padded_len(P);
     cplx<T>* buf = bufs + (size_t)g * 2 * PL;
     cplx<T>* buf2 = buf + PL;
-    const int64_t start = south ? rp.start_s : rp.start_n;
-    const int64_t foff = south ? rp.foff_s : rp.foff_n;
-    const int shift = south ? rp.shift_s : rp.shift_n;
-    const int64_t np = geo.npix;
-    const int b0 = blockIdx.y * maps_per_cta;
-    const int b1 = min(b0 + maps_per_cta, nmaps);
-    if (b1 > b0 && !(HPX_INB(b0 * np + start, kExtMap, 3) && HPX_INB((b1 - 1) * np + start + 2 * rp.h - 1, kExtMap, 3) &&
-                     HPX_INB(2 * ((int64_t)(b1 - 1) * Ftot + foff + rp.mt) - 1, kExtF, 4)))
-        return;
+    const int64_t np = a.geo.npix;
+    const RingItems<BOTH> it(rp, z, y, a.maps_per_cta, a.nmaps);
+    if (it.q1 > it.q0) {
+        const int b0 = it.map(it.q0), b1 = it.map(it.q1 - 1);
+        if (!(HPX_INB(b0 * np + it.start(it.q0), kExtMap, 3) &&
+              HPX_INB(b1 * np + it.start(it.q1 - 1) + 2 * rp.h - 1, kExtMap, 3) &&
+              HPX_INB(2 * ((int64_t)b1 * a.Ftot + it.foff(it.q1 - 1) + rp.mt) - 1, kExtF, 4)))
+            return;
+    }
     cplx<T>* cur = buf;
     cplx<T>* other = buf2;
-    auto spec = [&](int bb) { return (const cplx<T>*)(F + 2 * ((int64_t)bb * Ftot + foff)); };
-    if (b0 + g < b1) spec_load_async(cur, spec(b0 + g), rp.mt, lt, tpf);
-    for (int b = b0 + g; b < b1; b += S) {
+    auto spec = [&](int q) { return (const cplx<T>*)(F + 2 * ((int64_t)it.map(q) * a.Ftot + it.foff(q))); };
+    if (it.q0 + g < it.q1) spec_load_async(cur, spec(it.q0 + g), rp.mt, lt, tpf);
+    for (int q = it.q0 + g; q < it.q1; q += S) {
         auto load_next = [&](cplx<T>* dst) {
-            if (b + S < b1) spec_load_async(dst, spec(b + S), rp.mt, lt, tpf);
+            if (q + S < it.q1) spec_load_async(dst, spec(q + S), rp.mt, lt, tpf);
         };
-        ring_inverse<KIND>(cur, other, shift, map + (int64_t)b * np + start,
-                           ref ? ref + (int64_t)b * np + start : nullptr, rp, tw, Gs, cs, E, lt, tpf, g, load_next);
+        const int64_t o = (int64_t)it.map(q) * np + it.start(q);
+        ring_inverse<KIND>(cur, other, it.shift(q), map + o, ref ? ref + o : nullptr, rp, tw, Gs, cs, E, lt, tpf, g,
+                           load_next);
     }
+}
+
+template <typename T, int KIND, bool BOTH>
+__global__ void __launch_bounds__(ring_kernel_threads<KIND>(), ring_kernel_ctas<T, KIND>())
+    k_ring_inv(RingInvArgs a, const T* __restrict__ F, T* __restrict__ map, const cplx<T>* __restrict__ rtab,
+               const cplx<T>* __restrict__ gtab, const cplx<T>* __restrict__ chirp, const T* __restrict__ ref) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int2 c = ring_cta<KIND, BOTH>();
+    ring_inv_cta<T, KIND, BOTH>(smem_raw, a, c.x, blockIdx.y, c.y, F, map, rtab, gtab, chirp, ref);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, ring_kernel_ctas<T, 1>())
+    k_ring_inv_any(RingInvArgs a, int n_blue, int n_pow2, const T* __restrict__ F, T* __restrict__ map,
+                   const cplx<T>* __restrict__ rtab, const cplx<T>* __restrict__ gtab,
+                   const cplx<T>* __restrict__ chirp, const T* __restrict__ ref) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int x = blockIdx.x;
+    if (x < n_blue) ring_inv_cta<T, 1, true>(smem_raw, a, n_pow2 + x, blockIdx.y, 0, F, map, rtab, gtab, chirp, ref);
+    else ring_inv_cta<T, 0, true>(smem_raw, a, x - n_blue, blockIdx.y, 0, F, map, rtab, gtab, chirp, ref);
 }
 
 // Per-map max |a| over the coefficients the synthesis uses, a[b][l][m] for

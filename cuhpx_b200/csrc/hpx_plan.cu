@@ -95,7 +95,7 @@ struct hpx_plan_s {
     RingPair* d_pairs = nullptr;
     // ring lists of the three ring-kernel instantiations: power-of-two rings,
     // Bluestein rings of length 2^K, then of length 3 * 2^K (largest first
-    // within each), as ring indices t
+    // within each), as ring pairs
     int* d_rings = nullptr;
     int n_rings_pow2 = 0, n_rings_blue = 0, n_rings_blue3 = 0;
     int hblue = 0, pblue = 0;    // largest h and FFT length of the Bluestein rings of length 2^K
@@ -226,6 +226,17 @@ struct DeviceGuard {
     }
 };
 
+template <typename T>
+std::vector<const void*> ring_kernels() {
+    return {(const void*)k_ring_fwd_any<T>,        (const void*)k_ring_inv_any<T>,
+            (const void*)k_ring_fwd<T, 0, true>,   (const void*)k_ring_fwd<T, 1, true>,
+            (const void*)k_ring_fwd<T, 2, true>,   (const void*)k_ring_fwd<T, 0, false>,
+            (const void*)k_ring_fwd<T, 1, false>,  (const void*)k_ring_fwd<T, 2, false>,
+            (const void*)k_ring_inv<T, 0, true>,   (const void*)k_ring_inv<T, 1, true>,
+            (const void*)k_ring_inv<T, 2, true>,   (const void*)k_ring_inv<T, 0, false>,
+            (const void*)k_ring_inv<T, 1, false>,  (const void*)k_ring_inv<T, 2, false>};
+}
+
 // largest L the plans accept
 template <typename T>
 constexpr int max_degrees() { return sizeof(T) == 4 ? 12956 : 11420; }
@@ -325,12 +336,8 @@ int create_typed(hpx_plan_s* P) {
     HPX_CUDA_TRY(cudaStreamCreateWithFlags(&P->aux, cudaStreamNonBlocking));
     HPX_CUDA_TRY(cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming));
     HPX_CUDA_TRY(cudaEventCreateWithFlags(&P->ev_join, cudaEventDisableTiming));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_fwd<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_fwd<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_fwd<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_inv<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_inv<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_ring_inv<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
+    for (const void* f : ring_kernels<T>())
+        HPX_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     const int rc_direct = direct_attributes<T>(dev_max);
     if (rc_direct != HPX_OK) return rc_direct;
     HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_simt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
@@ -847,8 +854,8 @@ int plan_build(hpx_plan_s* P) {
     HPX_CUDA_TRY(cudaMemcpy(P->d_pairs, P->h_pairs.data(), sizeof(RingPair) * P->NP, cudaMemcpyHostToDevice));
     {
         std::vector<int> pw, bl, b3;
-        auto pair_of = [&](int t) -> const RingPair& { return P->h_pairs[t < P->NP ? t : P->R - 1 - t]; };
-        for (int t = 0; t < P->R; ++t) {
+        auto pair_of = [&](int p) -> const RingPair& { return P->h_pairs[p]; };
+        for (int t = 0; t < P->NP; ++t) {
             const RingPair& rp = pair_of(t);
             if (rp.logh >= 0) {
                 pw.push_back(t);
@@ -1059,10 +1066,37 @@ struct Pipeline {
         }
     };
 
-    // maps per ring CTA (default 16: amortises the CTA's table set-up -- phase
-    // and twiddle tables, Bluestein chirp tables -- over twice the maps of 8,
-    // 2.5% of the step; 32 measured no better); set by hpx_plan_set_schedule
-    int maps_per_cta_ring() const { return P->ring_g; }
+    // How the ring CTAs share a call's transforms: maps per CTA, and whether a CTA
+    // takes both rings of its pair (BOTH).
+    //   more than 16 maps: one ring, the schedule's maps per CTA (default 16:
+    //     amortises the CTA's table set-up -- phase and twiddle tables, Bluestein
+    //     chirp tables -- over twice the maps of 8, 2.5% of the step; 32 measured no
+    //     better);
+    //   up to 16: both rings of half as many maps, so that the set-up is
+    //     shared from the first map on (nside 1024, 8 maps: 459 / 510 us against
+    //     480 / 531), and fewer maps only while that leaves less than a CTA an SM (a
+    //     second wave costs more than it hides: nside 128, 4 maps FP64, 256 CTAs
+    //     20 / 21 us, 512 CTAs 28 / 28 us).
+    // Up to 1200 CTAs of the two common kinds of rings go out as one launch
+    // (k_ring_*_any) instead of two on forked streams: nside 32, one map 18.4 ->
+    // 14 us; with 4,096 CTAs the two streams are the faster (nside 256, 64 maps:
+    // 255 against 276 us), the power-of-two rings running three CTAs an SM there.
+    struct RingSplit {
+        int maps;
+        bool both, one_launch;
+        unsigned groups, sides;
+    };
+    RingSplit ring_split(int nb) const {
+        RingSplit r{};
+        r.both = nb <= 16;
+        r.sides = r.both ? 1 : 2;
+        r.maps = r.both ? std::max(1, P->ring_g / 2) : P->ring_g;
+        while (r.both && r.maps > 1 && (int64_t)P->NP * ((nb + r.maps - 1) / r.maps) < 148) r.maps >>= 1;
+        r.groups = (unsigned)((nb + r.maps - 1) / r.maps);
+        r.one_launch = r.both && P->n_rings_pow2 && P->n_rings_blue && !P->n_rings_blue3 &&
+                       (int64_t)P->NP * r.groups <= 1200;
+        return r;
+    }
 
     // The power-of-two rings on the plan's auxiliary stream and the Bluestein
     // rings (2^K, then 3072 points) on st, forked and joined by events (valid
@@ -1089,30 +1123,33 @@ struct Pipeline {
 
     // map -> ring spectra F
     void ring_fft_fwd(const T* map, int nb, unsigned* fmax) {
-        const int g = maps_per_cta_ring();
-        {
-            Timer tm(P, st, kStRingFwd);
-            if (fmax) cudaMemsetAsync(fmax, 0, sizeof(unsigned) * nb, st);
-            const unsigned nbk = (nb + g - 1) / g;
-            const cplx<T>* gt = (const cplx<T>*)P->d_gtab;
-            const cplx<T>* ch = (const cplx<T>*)P->d_chirp;
-            const cplx<T>* rt = (const cplx<T>*)P->d_rtab;
-            ring_launches(
-                [&](cudaStream_t s) {
-                    k_ring_fwd<T, 0><<<dim3(P->n_rings_pow2, nbk), 256, P->ring_smem, s>>>(
-                        map, nb, g, F, P->Ftot, P->geo, P->d_pairs, P->d_rings, rt, P->rslot, gt, ch, fmax);
-                },
-                [&](cudaStream_t s) {
-                    if (P->n_rings_blue)
-                        k_ring_fwd<T, 1><<<dim3(P->n_rings_blue, nbk), 256, P->blue_smem, s>>>(
-                            map, nb, g, F, P->Ftot, P->geo, P->d_pairs, P->d_rings + P->n_rings_pow2, rt, P->rslot, gt,
-                            ch, fmax);
-                    if (P->n_rings_blue3)
-                        k_ring_fwd<T, 2><<<dim3(P->n_rings_blue3, nbk), ring_kernel_threads<2>(), P->blue3_smem, s>>>(
-                            map, nb, g, F, P->Ftot, P->geo, P->d_pairs, P->d_rings + P->n_rings_pow2 + P->n_rings_blue,
-                            rt, P->rslot, gt, ch, fmax);
-                });
+        const RingSplit rs = ring_split(nb);
+        Timer tm(P, st, kStRingFwd);
+        if (fmax) cudaMemsetAsync(fmax, 0, sizeof(unsigned) * nb, st);
+        const cplx<T>* gt = (const cplx<T>*)P->d_gtab;
+        const cplx<T>* ch = (const cplx<T>*)P->d_chirp;
+        const cplx<T>* rt = (const cplx<T>*)P->d_rtab;
+        RingFwdArgs a{nb, rs.maps, P->Ftot, P->geo, P->d_pairs, P->d_rings, P->rslot, fmax};
+        if (rs.one_launch) {
+            k_ring_fwd_any<T><<<dim3(P->n_rings_blue + P->n_rings_pow2, rs.groups), 256, std::max(P->ring_smem, P->blue_smem),
+                                st>>>(a, P->n_rings_blue, P->n_rings_pow2, map, F, rt, gt, ch);
+            return;
         }
+        ring_launches(
+            [&](cudaStream_t s) {
+                (rs.both ? k_ring_fwd<T, 0, true> : k_ring_fwd<T, 0, false>)<<<dim3(P->n_rings_pow2 * rs.sides, rs.groups), 256,
+                    P->ring_smem, s>>>(a, map, F, rt, gt, ch);
+            },
+            [&](cudaStream_t s) {
+                a.rings = P->d_rings + P->n_rings_pow2;
+                if (P->n_rings_blue)
+                    (rs.both ? k_ring_fwd<T, 1, true> : k_ring_fwd<T, 1, false>)<<<dim3(P->n_rings_blue * rs.sides, rs.groups), 256,
+                    P->blue_smem, s>>>(a, map, F, rt, gt, ch);
+                a.rings += P->n_rings_blue;
+                if (P->n_rings_blue3)
+                    (rs.both ? k_ring_fwd<T, 2, true> : k_ring_fwd<T, 2, false>)<<<dim3(P->n_rings_blue3 * rs.sides, rs.groups), ring_kernel_threads<2>(),
+                    P->blue3_smem, s>>>(a, map, F, rt, gt, ch);
+            });
     }
     // map -> ring spectra F -> folded Legendre operand (spec, or bf16 hi/lo)
     void ring_fwd(const T* map, int nb, int adjoint) {
@@ -1135,26 +1172,31 @@ struct Pipeline {
     }
     // ring spectra F -> map
     void ring_fft_inv(T* map, int nb, const T* ref) {
-        const int g = maps_per_cta_ring();
+        const RingSplit rs = ring_split(nb);
         Timer tm(P, st, kStRingInv);
-        const unsigned nbk = (nb + g - 1) / g;
         const cplx<T>* gt = (const cplx<T>*)P->d_gtab;
         const cplx<T>* ch = (const cplx<T>*)P->d_chirp;
         const cplx<T>* rt = (const cplx<T>*)P->d_rtab;
+        RingInvArgs a{nb, rs.maps, P->Ftot, P->geo, P->d_pairs, P->d_rings, P->rslot};
+        if (rs.one_launch) {
+            k_ring_inv_any<T><<<dim3(P->n_rings_blue + P->n_rings_pow2, rs.groups), 256, std::max(P->ring_smem, P->blue_smem),
+                                st>>>(a, P->n_rings_blue, P->n_rings_pow2, F, map, rt, gt, ch, ref);
+            return;
+        }
         ring_launches(
             [&](cudaStream_t s) {
-                k_ring_inv<T, 0><<<dim3(P->n_rings_pow2, nbk), 256, P->ring_smem, s>>>(
-                    F, P->Ftot, map, nb, g, P->geo, P->d_pairs, P->d_rings, rt, P->rslot, gt, ch, ref);
+                (rs.both ? k_ring_inv<T, 0, true> : k_ring_inv<T, 0, false>)<<<dim3(P->n_rings_pow2 * rs.sides, rs.groups), 256,
+                    P->ring_smem, s>>>(a, F, map, rt, gt, ch, ref);
             },
             [&](cudaStream_t s) {
+                a.rings = P->d_rings + P->n_rings_pow2;
                 if (P->n_rings_blue)
-                    k_ring_inv<T, 1><<<dim3(P->n_rings_blue, nbk), 256, P->blue_smem, s>>>(
-                        F, P->Ftot, map, nb, g, P->geo, P->d_pairs, P->d_rings + P->n_rings_pow2, rt, P->rslot,
-                        gt, ch, ref);
+                    (rs.both ? k_ring_inv<T, 1, true> : k_ring_inv<T, 1, false>)<<<dim3(P->n_rings_blue * rs.sides, rs.groups), 256,
+                    P->blue_smem, s>>>(a, F, map, rt, gt, ch, ref);
+                a.rings += P->n_rings_blue;
                 if (P->n_rings_blue3)
-                    k_ring_inv<T, 2><<<dim3(P->n_rings_blue3, nbk), ring_kernel_threads<2>(), P->blue3_smem, s>>>(
-                        F, P->Ftot, map, nb, g, P->geo, P->d_pairs, P->d_rings + P->n_rings_pow2 + P->n_rings_blue,
-                        rt, P->rslot, gt, ch, ref);
+                    (rs.both ? k_ring_inv<T, 2, true> : k_ring_inv<T, 2, false>)<<<dim3(P->n_rings_blue3 * rs.sides, rs.groups), ring_kernel_threads<2>(),
+                    P->blue3_smem, s>>>(a, F, map, rt, gt, ch, ref);
             });
     }
     // The contraction that reads and writes the ring spectra itself

@@ -229,7 +229,9 @@ HPX_API int hpx_plan_create_latlon(const hpx_latlon_desc_t* desc, hpx_plan_t* pl
 /* Launch schedule of a plan (no counterpart in cuHPX, whose einsum and cuFFT
  * calls have none): the autotuner of this library (cuhpx_b200/autotune.py)
  * times candidates and keeps the fastest per GPU and problem.
- *   ring_maps_per_cta  maps each ring-FFT CTA transforms (4, 8, 16 or 32; 16)
+ *   ring_maps_per_cta  rings each ring-FFT CTA transforms (4, 8, 16 or 32; 16): one
+ *                      ring of that many maps, or, in calls of up to 16 maps, both
+ *                      rings of a pair of half as many
  *   fwd_deal, inv_deal how the persistent tensor-core kernels' tiles are dealt
  *                      to their CTAs (the m-to-CTA schedule), HPX_DEAL_*
  *   ctas               persistent CTAs of those kernels (0: one per SM)
