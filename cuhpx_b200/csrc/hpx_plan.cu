@@ -36,6 +36,7 @@
 #include "../../include/hpx_b200.h"
 #include "hpx_kernels.cuh"
 #include "legendre_direct.cuh"
+#include "legendre_tile.cuh"
 #include "legendre_tc.cuh"
 #include "hpx_remap.cuh"
 #include "hpx_healpy.cuh"
@@ -195,7 +196,10 @@ struct hpx_plan_s {
     int cols() const { return ((2 * batch_chunk) + 3) & ~3; }
     size_t spec_bytes() const { return (size_t)M * 2 * NP * cols() * real_size(); }
     // order-major analysis output of the tensor cores where the ring spectra cannot hold it
-    size_t almT_bytes() const { return mixed() ? (size_t)M * L * cols() * real_size() : 0; }
+    // (mixed plans), or the tiled FP32 synthesis' coefficient columns
+    size_t almT_bytes() const { return mixed() || tiled() ? (size_t)M * L * cols() * real_size() : 0; }
+    // plans whose chunks can take the tiled FP32 contractions (legendre_tile.cuh)
+    bool tiled() const { return prec == HPX_PREC_FP32; }
     size_t resid_bytes() const { return (size_t)batch_chunk * npix * real_size(); }
     size_t F_bytes() const { return (size_t)batch_chunk * Ftot * 2 * real_size(); }
     bool mixed() const { return prec == HPX_PREC_BF16X3 || prec == HPX_PREC_F16X3; }
@@ -256,6 +260,8 @@ cudaError_t vec_attribute(int bytes) {
 }
 template <typename T>
 int direct_attributes(int dev_max) {
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileFwdSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileInvSmem));
     HPX_CUDA_TRY((vec_attribute<T, 1, 2>(dev_max)));
     HPX_CUDA_TRY((vec_attribute<T, 1, 4>(dev_max)));
     HPX_CUDA_TRY((vec_attribute<T, 2, 2>(dev_max)));
@@ -325,7 +331,7 @@ int create_typed(hpx_plan_s* P) {
     // of buffers, within ring_smem_elems' 2 x 4096)
     P->blue3_smem =
         P->n_rings_blue3 ? (ring_smem_elems(P->bufP, P->nmax) + P->pblue3 / 2 + 2 + P->hblue3) * sizeof(C) : 0;
-    P->fwd_smem = fwd_smem_bytes<T>();
+    if (P->f64) P->fwd_smem = fwd_smem_bytes<T>();
     int dev_max = 0;
     HPX_CUDA_TRY(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device));
     if ((int)P->ring_smem > dev_max || (int)P->blue_smem > dev_max || (int)P->blue3_smem > dev_max ||
@@ -340,7 +346,8 @@ int create_typed(hpx_plan_s* P) {
         HPX_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     const int rc_direct = direct_attributes<T>(dev_max);
     if (rc_direct != HPX_OK) return rc_direct;
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_simt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
+    if constexpr (sizeof(T) == 8)
+        HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_simt<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_max));
     return HPX_OK;
 }
 
@@ -1199,13 +1206,12 @@ struct Pipeline {
                     P->blue3_smem, s>>>(a, F, map, rt, gt, ch, ref);
             });
     }
-    // The contraction that reads and writes the ring spectra itself
-    // (legendre_direct.cuh): every FP32 and FP64 synthesis (nside 512, 64 maps:
-    // 4.6 ms against 6.3 ms of the tiled kernel it replaced, with its layout
-    // and unfold launches) and the analysis of up to 36 maps (FP32, nside 256: 32
-    // maps 708 us against 789 us tiled with the fold, 48 maps 987 against 878;
-    // FP64 crosses over there too: 32 maps 2003 against 1977 us).
-    bool direct_fwd(int nb) const { return !P->mixed() && nb <= (sizeof(T) == 4 ? 36 : 30); }
+    // The contractions that read and write the ring spectra themselves
+    // (legendre_direct.cuh): FP32 wherever the tiled ones are not the better,
+    // FP64 synthesis always (nside 256, 32 maps: 957 us against 2583 us of the tiled
+    // kernel it replaced) and FP64 analysis up to 30 maps (nside 256: 16 maps 1107
+    // us against 1793 tiled, 32 maps 2003 against 1977).
+    bool direct_fwd(int nb) const { return !P->mixed() && (sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 30); }
     const typename DirRec<T>::Coef* dir_coef() const {
         if constexpr (sizeof(T) == 4) return P->d_alpha;
         else return P->d_coef;
@@ -1306,9 +1312,31 @@ struct Pipeline {
             leg_fwd(alm, nb, accumulate);
         }
     }
+    void leg_inv_tile(const float* alm, int nb) {
+        const int C = P->cols();
+        {
+            Timer tm(P, st, kStAlmCols);
+            k_alm_to_tile<<<dim3((P->M + 31) / 32, P->L, (nb + 63) / 64), 256, 0, st>>>(alm, nb, P->L, P->M, P->d_norm,
+                                                                                     P->Lpad, (float*)almT, C);
+        }
+        Timer tm(P, st, kStLegInv);
+        k_leg_inv_tile<<<dim3((P->NP + kTileInvRing - 1) / kTileInvRing, P->M, (2 * nb + kTileCols - 1) / kTileCols),
+                         kTileThreads, kTileInvSmem, st>>>((const float*)almT, C, (float*)spec, P->L, P->M, P->geo, P->d_z,
+                                                           P->d_lstart, P->d_pstart, P->d_alpha, P->d_norm, P->Lpad);
+    }
+    // The tiled FP32 contractions (legendre_tile.cuh) against the direct ones, whole
+    // calls: analysis nside 256, 32 maps 667 / 694 us, 16 maps 613 / 411; nside
+    // 128, 32 maps 161 / 156, 48 maps 185 / 227; below that the three launches
+    // more decide (nside 64, 48 maps 67 / 66, 64 maps 75 / 77).  Synthesis nside 512, 48
+    // maps 4200 / 4531, 32 maps 3754 / 3044; nside 128, 64 maps 207 / 221.
+    bool tile_fwd(int nb) const { return P->tiled() && nb > (P->NP >= 256 ? 30 : 56); }
+    bool tile_inv(int nb) const { return P->tiled() && P->NP >= 256 && nb > (P->NP >= 512 ? 46 : 56); }
     // alm -> map (ref: residual ref - map)
     void synthesis(const T* alm, T* map, int nb, int adjoint, const T* ref) {
-        if (!P->mixed()) {
+        if (tile_inv(nb)) {
+            if constexpr (sizeof(T) == 4) leg_inv_tile(alm, nb);
+            ring_inv(map, nb, adjoint, ref);
+        } else if (!P->mixed()) {
             leg_inv_direct(alm, nb, adjoint);
             ring_fft_inv(map, nb, ref);
         } else {
@@ -1343,10 +1371,17 @@ struct Pipeline {
             return;
         }
         Timer tm(P, st, kStLegFwd);
-        dim3 grid(P->n_fwdtiles, (C + FwdCfg<T>::CT - 1) / FwdCfg<T>::CT);
-        k_leg_fwd_simt<T><<<grid, 256, P->fwd_smem, st>>>(spec, C, nb, alm, P->L, P->M, P->geo, P->d_pairs,
-                                                          P->d_lstart, P->d_pstart, P->d_coef, P->Lpad, P->d_seeds,
-                                                          P->d_fwdtiles, accumulate);
+        if constexpr (sizeof(T) == 4) {
+            const int nj = (P->L + kTileDeg - 1) / kTileDeg, nt = (P->M + 3) / 4 * 4 * nj;
+            k_leg_fwd_tile<<<dim3(nt + (accumulate ? 0 : 148), (C + kTileCols - 1) / kTileCols), kTileThreads,
+                             kTileFwdSmem, st>>>(spec, C, nb, alm, P->L, P->M, P->geo, P->d_z, P->d_lstart, P->d_pstart,
+                                                 P->d_alpha, P->d_norm, P->Lpad, P->d_seeds, nj, nt, accumulate);
+        } else {
+            dim3 grid(P->n_fwdtiles, (C + FwdCfg<T>::CT - 1) / FwdCfg<T>::CT);
+            k_leg_fwd_simt<T><<<grid, 256, P->fwd_smem, st>>>(spec, C, nb, alm, P->L, P->M, P->geo, P->d_pairs,
+                                                              P->d_lstart, P->d_pstart, P->d_coef, P->Lpad, P->d_seeds,
+                                                              P->d_fwdtiles, accumulate);
+        }
     }
     void leg_inv(const T* alm, int nb) {
         const int C = P->cols();
