@@ -319,22 +319,24 @@ __global__ void __launch_bounds__(256) k_alm_maxabs(const float* __restrict__ al
 // Output spec[m][par][p][col] in T, or hi/lo pairs xh/xl (mixed plans): bf16,
 // or, with fmax given, fp16 of the values times 2^e(map), e from the map's
 // max |F| (recorded by k_ring_fwd) times the bound wb on |c| (F_t + F_t').
-// CTA per (block of 32 orders, ring pair); the transpose goes through shared memory.
-template <typename T>
-constexpr int fold_mb() { return sizeof(T) == 4 ? 32 : 16; }
+// Rows are C wide, of which ncols are columns (hi and lo packed into one row: C = 2
+// ncols, xl = xh + ncols / 2).  CTA per (block of orders, ring pair, NB = 64 or 16
+// maps); the transpose goes through shared memory.
+template <typename T, int NB>
+constexpr int fold_mb() { return (sizeof(T) == 4 ? 2048 : 1024) / NB; }
 
-template <typename T>
+template <typename T, int NB>
 __global__ void __launch_bounds__(256) k_fold(const T* __restrict__ F, int64_t Ftot, int nmaps, Geom geo,
                                               const RingPair* __restrict__ pairs, int adjoint, T* __restrict__ spec,
-                                              int C, uint32_t* __restrict__ xh, uint32_t* __restrict__ xl,
+                                              int C, int ncols, uint32_t* __restrict__ xh, uint32_t* __restrict__ xl,
                                               const unsigned* __restrict__ fmax, float wb) {
-    constexpr int MB = fold_mb<T>();
-    constexpr int NL = 64 * MB / 256;  // elements per thread (the kernel runs 256 threads)
-    __shared__ cplx<T> tn[64][MB + 1];
-    __shared__ cplx<T> ts[64][MB + 1];
-    __shared__ float s_sc[64];
+    constexpr int MB = fold_mb<T, NB>();
+    constexpr int NL = NB * MB / 256;  // elements per thread (the kernel runs 256 threads)
+    __shared__ cplx<T> tn[NB][MB + 1];
+    __shared__ cplx<T> ts[NB][MB + 1];
+    __shared__ float s_sc[NB];
     const int NP = geo.NP;
-    const int m0 = blockIdx.x * MB, p = blockIdx.y, bz = blockIdx.z * 64;
+    const int m0 = blockIdx.x * MB, p = blockIdx.y, bz = blockIdx.z * NB;
     const RingPair rp = pairs[p];
     if (m0 >= rp.mt) return;
     const int tid = threadIdx.x;
@@ -353,7 +355,7 @@ __global__ void __launch_bounds__(256) k_fold(const T* __restrict__ F, int64_t F
                 vs[k] = *(const cplx<T>*)(F + 2 * ((int64_t)b * Ftot + rp.foff_s + m));
         }
     }
-    if (xh && fmax && tid < 64) {
+    if (xh && fmax && tid < NB) {
         // FP16 operands scaled by 2^e(map); |S|, |D| <= wb * max|F|
         const int b = bz + tid;
         s_sc[tid] = tc::pow2f(tc::f16_scale_exp(__uint_as_float(b < nmaps ? fmax[b] : 0u) * wb));
@@ -369,8 +371,8 @@ __global__ void __launch_bounds__(256) k_fold(const T* __restrict__ F, int64_t F
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const int i = tid + 256 * k;
-        const int mm = i >> 6, bl = i & 63, b = bz + bl, m = m0 + mm;
-        if (m >= rp.mt || 2 * b >= C) continue;
+        const int mm = i / NB, bl = i % NB, b = bz + bl, m = m0 + mm;
+        if (m >= rp.mt || 2 * b >= ncols) continue;
         const T wk = adjoint ? ((m == 0 || m == rp.h) ? (T)1 : (T)2) : (T)rp.w;
         const cplx<T> a = tn[bl][mm], c = ts[bl][mm];
         cplx<T> S, D;
@@ -417,16 +419,16 @@ __global__ void __launch_bounds__(256) k_fold(const T* __restrict__ F, int64_t F
 // Unfold the synthesis output spec[m][par][p][col] (E = even, O = odd degrees)
 // into ring spectra F_t = sc (E + O), F_t' = sc (E - O), with sc = 1, or for
 // the adjoint of analysis sc = w_t (m = 0, nphi/2) and w_t/2 otherwise.
-template <typename T>
+template <typename T, int NB>
 __global__ void __launch_bounds__(256) k_unfold(const T* __restrict__ spec, int C, int nmaps, Geom geo,
                                                 const RingPair* __restrict__ pairs, int adjoint, T* __restrict__ F,
                                                 int64_t Ftot) {
-    constexpr int MB = fold_mb<T>();
-    constexpr int NL = 64 * MB / 256;  // elements per thread (the kernel runs 256 threads)
-    __shared__ cplx<T> te[MB][65];
-    __shared__ cplx<T> to[MB][65];
+    constexpr int MB = fold_mb<T, NB>();
+    constexpr int NL = NB * MB / 256;  // elements per thread (the kernel runs 256 threads)
+    __shared__ cplx<T> te[MB][NB + 1];
+    __shared__ cplx<T> to[MB][NB + 1];
     const int NP = geo.NP;
-    const int m0 = blockIdx.x * MB, p = blockIdx.y, bz = blockIdx.z * 64;
+    const int m0 = blockIdx.x * MB, p = blockIdx.y, bz = blockIdx.z * NB;
     const RingPair rp = pairs[p];
     if (m0 >= rp.mt) return;
     const int tid = threadIdx.x;
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(256) k_unfold(const T* __restrict__ spec, int 
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const int i = tid + 256 * k;
-        const int mm = i >> 6, bl = i & 63, b = bz + bl, m = m0 + mm;
+        const int mm = i / NB, bl = i % NB, b = bz + bl, m = m0 + mm;
         ve[k] = {(T)0, (T)0};
         vo[k] = {(T)0, (T)0};
         if (m < rp.mt && 2 * b < C && HPX_INB((((int64_t)m * 2 + 1) * NP + p) * C + 2 * b + 1, kExtSpec, 7)) {
@@ -446,8 +448,8 @@ __global__ void __launch_bounds__(256) k_unfold(const T* __restrict__ spec, int 
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const int i = tid + 256 * k;
-        te[i >> 6][i & 63] = ve[k];
-        to[i >> 6][i & 63] = vo[k];
+        te[i / NB][i % NB] = ve[k];
+        to[i / NB][i % NB] = vo[k];
     }
     __syncthreads();
 #pragma unroll

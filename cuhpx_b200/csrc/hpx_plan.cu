@@ -601,14 +601,18 @@ int tc_create(hpx_plan_s* P) {
     }
     const int rc_deal = tc_deal(P, HPX_DEAL_ORDER_SNAKE, HPX_DEAL_ORDER_SNAKE, 0);
     if (rc_deal != HPX_OK) return rc_deal;
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
-    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_fwd_tc<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
+    HPX_CUDA_TRY(cudaFuncSetAttribute(k_leg_inv_tc<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kISmem));
     T.active = 1;
     return HPX_OK;
 }
@@ -617,8 +621,8 @@ int tc_create(hpx_plan_s* P) {
 // [outer][rows][128 cols] with a {64 cols, box_rows} box, 128B swizzle.
 // spec[2M][NP][C] (FP32) for the synthesis epilogue's TMA stores: boxes of
 // 16 columns x 32 rings in the 64-byte swizzle
-int encode_spec_store(const hpx_plan_s* P, CUtensorMap* map, void* spec) {
-    const cuuint64_t C = (cuuint64_t)P->cols();
+int encode_spec_store(const hpx_plan_s* P, CUtensorMap* map, void* spec, int cols) {
+    const cuuint64_t C = (cuuint64_t)cols;
     const cuuint64_t dims[3] = {C, (cuuint64_t)P->NP, 2ull * P->M};
     const cuuint64_t strides[2] = {C * 4, C * 4 * P->NP};
     const cuuint32_t box[3] = {16, 32, 1};
@@ -630,9 +634,10 @@ int encode_spec_store(const hpx_plan_s* P, CUtensorMap* map, void* spec) {
     return HPX_OK;
 }
 
-int encode_operand(const hpx_plan_s* P, CUtensorMap* map, void* base, uint64_t rows, uint64_t outer, int box_rows) {
-    const cuuint64_t dims[3] = {(cuuint64_t)kTcCols, rows, outer};
-    const cuuint64_t strides[2] = {(cuuint64_t)kTcCols * 2, (cuuint64_t)kTcCols * 2 * rows};
+int encode_operand(const hpx_plan_s* P, CUtensorMap* map, void* base, uint64_t rows, uint64_t outer, int box_rows,
+                   int cols) {
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, rows, outer};
+    const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)cols * 2 * rows};
     const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
     const cuuint32_t es[3] = {1, 1, 1};
     CUresult r = ((EncodeTiledFn)P->tc.encode)(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, es,
@@ -1158,22 +1163,41 @@ struct Pipeline {
                     P->blue3_smem, s>>>(a, map, F, rt, gt, ch);
             });
     }
+    // Tensor-core calls of up to kPkMaps maps on the resident table take packed
+    // operand rows and 32 result columns instead of 128 (legendre_tc.cuh).
+    bool packed(int nb) const { return P->mixed() && P->tc.table && nb <= kPkMaps; }
+    int spec_cols(int nb) const { return packed(nb) ? kPkCols : P->cols(); }
+    template <int NB>
+    dim3 fold_grid(int nb) const {
+        constexpr int MB = fold_mb<T, NB>();
+        return dim3((P->mtmax + MB - 1) / MB, P->NP, (nb + NB - 1) / NB);
+    }
     // map -> ring spectra F -> folded Legendre operand (spec, or bf16 hi/lo)
     void ring_fwd(const T* map, int nb, int adjoint) {
         ring_fft_fwd(map, nb, fmax);
         Timer tm(P, st, kStFold);
         // |c (F_t +- F_t')| <= 2 max|c| max|F|: c = w_t, or c_m <= 2 for the adjoint
         fold_wb = adjoint ? 4.f : 2.f * P->wmax;
-        dim3 fg((P->mtmax + fold_mb<T>() - 1) / fold_mb<T>(), P->NP, (nb + 63) / 64);
-        k_fold<T><<<fg, 256, 0, st>>>(F, P->Ftot, nb, P->geo, P->d_pairs, adjoint, spec, P->cols(), xh(), xl(),
-                                      fmax, fold_wb);
+        if (packed(nb)) {
+            if constexpr (sizeof(T) == 4)
+                k_fold<T, kPkMaps><<<fold_grid<kPkMaps>(nb), 256, 0, st>>>(F, P->Ftot, nb, P->geo, P->d_pairs, adjoint, spec,
+                                                                          2 * kPkCols, kPkCols, xh(), xh() + kPkCols / 2,
+                                                                          fmax, fold_wb);
+            return;
+        }
+        k_fold<T, 64><<<fold_grid<64>(nb), 256, 0, st>>>(F, P->Ftot, nb, P->geo, P->d_pairs, adjoint, spec, P->cols(),
+                                                        P->cols(), xh(), xl(), fmax, fold_wb);
     }
     // synthesis output spec (E/O) -> ring spectra F -> map (ref: residual ref - map)
     void ring_inv(T* map, int nb, int adjoint, const T* ref) {
         {
             Timer tm(P, st, kStUnfold);
-            dim3 fg((P->mtmax + fold_mb<T>() - 1) / fold_mb<T>(), P->NP, (nb + 63) / 64);
-            k_unfold<T><<<fg, 256, 0, st>>>(spec, P->cols(), nb, P->geo, P->d_pairs, adjoint, F, P->Ftot);
+            const int C = spec_cols(nb);
+            if (packed(nb))
+                k_unfold<T, kPkMaps><<<fold_grid<kPkMaps>(nb), 256, 0, st>>>(spec, C, nb, P->geo, P->d_pairs, adjoint, F,
+                                                                            P->Ftot);
+            else
+                k_unfold<T, 64><<<fold_grid<64>(nb), 256, 0, st>>>(spec, C, nb, P->geo, P->d_pairs, adjoint, F, P->Ftot);
         }
         ring_fft_inv(map, nb, ref);
     }
@@ -1348,6 +1372,7 @@ struct Pipeline {
         const int C = P->cols();
         if (P->mixed()) {
             const TcPlan& TP = P->tc;
+            const bool pk = packed(nb);
             float* yc = (float*)(P->ycols_in_F() ? (void*)F : (void*)ycols_alt);
             {
                 Timer tm(P, st, kStLegFwd);
@@ -1356,10 +1381,13 @@ struct Pipeline {
                 if (TP.n_fwd_tiles == 0) return;
                 CUtensorMap mh, ml;
                 const int box_rings = TP.table ? kFRingS<true> : kFRingS<false>;
-                if ((rc = encode_operand(P, &mh, xh(), P->NP, 2ull * P->M, box_rings)) != HPX_OK) return;
-                if ((rc = encode_operand(P, &ml, xl(), P->NP, 2ull * P->M, box_rings)) != HPX_OK) return;
-                auto kern = TP.table ? (P->f16() ? k_leg_fwd_tc<true, true> : k_leg_fwd_tc<false, true>)
-                                     : (P->f16() ? k_leg_fwd_tc<true, false> : k_leg_fwd_tc<false, false>);
+                if ((rc = encode_operand(P, &mh, xh(), P->NP, 2ull * P->M, box_rings, pk ? 2 * kPkCols : kTcCols)) != HPX_OK)
+                    return;
+                ml = mh;
+                if (!pk && (rc = encode_operand(P, &ml, xl(), P->NP, 2ull * P->M, box_rings, kTcCols)) != HPX_OK) return;
+                auto kern = pk         ? (P->f16() ? k_leg_fwd_tc<true, true, true> : k_leg_fwd_tc<false, true, true>)
+                        : TP.table ? (P->f16() ? k_leg_fwd_tc<true, true, false> : k_leg_fwd_tc<false, true, false>)
+                                     : (P->f16() ? k_leg_fwd_tc<true, false, false> : k_leg_fwd_tc<false, false, false>);
                 kern<<<TP.n_fwd_ctas, kTcThreads, kFSmem, st>>>(
                     mh, ml, TP.table ? TP.tab_fwd : mh, nb, yc, P->L, P->Lpad, P->geo, P->d_z, P->d_lstart,
                     P->d_lsmax, P->d_pstart, P->d_coef, P->d_alphac, P->d_seeds, TP.d_fwd_tiles, TP.d_fwd_off, fmax,
@@ -1367,7 +1395,7 @@ struct Pipeline {
             }
             Timer tm(P, st, kStColsAlm);
             dim3 tg((TP.m_tc_end + 31) / 32, P->L);
-            k_tc_to_alm<<<tg, dim3(32, 8), 0, st>>>(yc, nb, P->L, P->M, TP.m_tc_end, (float*)alm, accumulate);
+            (pk ? k_tc_to_alm<kPkMaps> : k_tc_to_alm<64>)<<<tg, dim3(32, 8), 0, st>>>(yc, nb, P->L, P->M, TP.m_tc_end, (float*)alm, accumulate);
             return;
         }
         Timer tm(P, st, kStLegFwd);
@@ -1384,7 +1412,8 @@ struct Pipeline {
         }
     }
     void leg_inv(const T* alm, int nb) {
-        const int C = P->cols();
+        const bool pk = packed(nb);
+        const int C = spec_cols(nb);
         const TcPlan& TP = P->tc;
         uint16_t* ah = tcA;
         uint16_t* al = tcA + (size_t)2 * P->M * TP.Lh * kTcCols;
@@ -1395,7 +1424,9 @@ struct Pipeline {
                 k_alm_maxabs<<<dim3((P->L + 7) / 8, nb), 256, 0, st>>>((const float*)alm, P->L, P->M, amax);
             }
             dim3 tg((P->M + 31) / 32, P->L + 64);
-            k_alm_to_tc<<<tg, dim3(32, 8), 0, st>>>((const float*)alm, nb, P->L, P->M, TP.Lh, ah, al, amax);
+            if (pk) al = ah + kPkCols;  // packed rows
+            (pk ? k_alm_to_tc<kPkMaps> : k_alm_to_tc<64>)<<<tg, dim3(32, 8), 0, st>>>((const float*)alm, nb, P->L, P->M,
+                                                                                     TP.Lh, ah, al, amax);
         }
         Timer tm(P, st, kStLegInv);
         // orders the tensor cores do not visit must read as zero in the ring stage
@@ -1404,12 +1435,14 @@ struct Pipeline {
                             (size_t)(P->M - TP.m_tc_end) * 2 * P->NP * C * sizeof(T), st);
         if (TP.n_inv_tiles == 0) return;
         CUtensorMap mh, ml;
-        if ((rc = encode_operand(P, &mh, ah, TP.Lh, 2ull * P->M, 32)) != HPX_OK) return;
-        if ((rc = encode_operand(P, &ml, al, TP.Lh, 2ull * P->M, 32)) != HPX_OK) return;
+        if ((rc = encode_operand(P, &mh, ah, TP.Lh, 2ull * P->M, 32, pk ? 2 * kPkCols : kTcCols)) != HPX_OK) return;
+        ml = mh;
+        if (!pk && (rc = encode_operand(P, &ml, al, TP.Lh, 2ull * P->M, 32, kTcCols)) != HPX_OK) return;
         CUtensorMap sm = mh;
-        if (TP.table && (rc = encode_spec_store(P, &sm, spec)) != HPX_OK) return;
-        auto kern = TP.table ? (P->f16() ? k_leg_inv_tc<true, true> : k_leg_inv_tc<false, true>)
-                             : (P->f16() ? k_leg_inv_tc<true, false> : k_leg_inv_tc<false, false>);
+        if (TP.table && (rc = encode_spec_store(P, &sm, spec, C)) != HPX_OK) return;
+        auto kern = pk         ? (P->f16() ? k_leg_inv_tc<true, true, true> : k_leg_inv_tc<false, true, true>)
+                        : TP.table ? (P->f16() ? k_leg_inv_tc<true, true, false> : k_leg_inv_tc<false, true, false>)
+                             : (P->f16() ? k_leg_inv_tc<true, false, false> : k_leg_inv_tc<false, false, false>);
         kern<<<TP.n_inv_ctas, kTcThreads, kISmem, st>>>(
             mh, ml, TP.table ? TP.tab_inv : mh, sm, (float*)spec, C, nb, P->L, P->M, P->Lpad, P->geo, P->d_z, P->d_lstart, P->d_lsmax,
             P->d_pstart, P->d_coef, P->d_alphac, P->d_seeds, TP.d_inv_tiles, TP.d_inv_off, amax, TP.d_err);

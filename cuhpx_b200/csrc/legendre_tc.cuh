@@ -152,6 +152,19 @@ __device__ __forceinline__ void epi_store_block(float* stg, const float (&v)[16]
     __syncwarp();
 }
 
+// Few maps (table-driven kernels, up to kPkMaps maps): an operand row packs the hi
+// and lo halves of 32 columns, [hi 32 | lo 32], one 128-byte swizzled row.  One
+// box then brings both, hi(A) x [hi | lo](B) gives the main and the first cross
+// product in one N = 64 MMA, and lo(A) x [hi | lo] issued 32 columns further adds
+// the second cross product (and lo x lo into columns nobody reads).  A quarter
+// of the operand bytes, of the output rows and of the layout work of 128 columns.
+constexpr int kPkMaps = 16, kPkCols = 2 * kPkMaps;
+constexpr int kPkStageBytes = 32768 + 8192;  // table part and operand part of a stage, both directions
+constexpr int kPkStages = 4;
+constexpr int kPkTmem = 128;                 // TMEM columns between the two parities
+template <bool PK>
+constexpr int kTcN = PK ? kPkCols : kTcCols;  // columns of a result row
+
 // Host-side state of the tensor-core path, owned by the plan.
 struct TcPlan {
     int active = 0;
@@ -469,7 +482,7 @@ __global__ void __launch_bounds__(64) k_table_first_nz(const uint16_t* __restric
 // producer groups than stages an mbarrier parity wait could pass on a stale
 // phase).  Lane = (ring r = lane&15, block pair bp = lane>>4) runs the two
 // blocks 2bp, 2bp+1 of its ring.
-template <bool F16, bool TAB>
+template <bool F16, bool TAB, bool PK>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_leg_fwd_tc(const __grid_constant__ CUtensorMap xh_map, const __grid_constant__ CUtensorMap xl_map,
                  const __grid_constant__ CUtensorMap tab_map, int nmaps,
@@ -478,6 +491,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                  const double2* __restrict__ coef, const AlphaC* __restrict__ alphac, const double2* __restrict__ seeds,
                  const int2* __restrict__ tiles, const int* __restrict__ tile_off, const unsigned* __restrict__ fmax,
                  float wb, int* __restrict__ err) {
+    static_assert(TAB || !PK, "packed operands go with the resident table");
     __shared__ float s_inv[kTcCols / 2];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // align by pointer arithmetic on the shared array (keeps the shared address space known)
@@ -490,11 +504,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int nbk = seed_blocks(L);
     const int t_begin = tile_off[blockIdx.x], t_end = tile_off[blockIdx.x + 1];  // this CTA's tiles
     load_inv_scales<F16>(s_inv, fmax, wb, nmaps);
-    tc_setup(sh, kFStagesS<TAB>, 1, warp, kEpiWarps<TAB>);
+    tc_setup(sh, PK ? kPkStages : kFStagesS<TAB>, 1, warp, kEpiWarps<TAB>);
     const uint32_t tmem = sh->tmem_base;
-    constexpr int RS = kFRingS<TAB>, NS = kFStagesS<TAB>, SB = kFStageBytesS<TAB>;
-    // stage s: A (Pbar) at s SB, B (operand) at s SB + SB/2; within each, the
-    // (par, hl) blocks are SB/8 apart and their two 64-wide halves SB/16 apart
+    constexpr int RS = kFRingS<TAB>, NS = PK ? kPkStages : kFStagesS<TAB>, SB = PK ? kPkStageBytes : kFStageBytesS<TAB>;
+    // stage s: A (Pbar) at s SB, B (operand) at s SB + SA; within each, the
+    // (par, hl) blocks are BL apart and their two 64-wide halves BL/2 apart
+    // (packed operand: one 64-wide block of BL/2 per parity)
+    constexpr int SA = PK ? 32768 : SB / 2, BL = SA / 4, NC = kTcN<PK>;
     auto nchunks = [&](int m) { return (NP - geo.first_ring(m) + RS - 1) / RS; };
 
     if (warp == 0) {
@@ -510,8 +526,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 for (int c = c0; c < nch; ++c, ++it) {
                     const int s = it % NS;
                     if (!tc::mbar_wait(&sh->empty[s], ((it / NS) & 1) ^ 1, err, 11)) goto tma_done;
-                    unsigned char* st = stages + s * SB + SB / 2;
-                    tc::mbar_arrive_tx(&sh->full_tma[s], TAB ? SB : SB / 2);
+                    unsigned char* st = stages + s * SB + SA;
+                    tc::mbar_arrive_tx(&sh->full_tma[s], TAB ? SB : SB - SA);
                     if (kWithholdTmaLoads) continue;
                     const int y = t0 + c * RS;  // rings past NP read as zeros (TMA out-of-bounds fill)
                     if (TAB) {
@@ -520,16 +536,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         for (int ph = 0; ph < 4; ++ph)
 #pragma unroll
                             for (int h = 0; h < 2; ++h)
-                                tc::tma_load_3d(stages + s * SB + ph * (SB / 8) + h * (SB / 16), &tab_map,
+                                tc::tma_load_3d(stages + s * SB + ph * BL + h * (BL / 2), &tab_map,
                                                 jb * (kTcFwdDeg / 2) + h * 64, y, 4 * m + ph, &sh->full_tma[s]);
+                    }
+                    if constexpr (PK) {
+#pragma unroll
+                        for (int par = 0; par < 2; ++par)
+                            tc::tma_load_3d(st + par * (BL / 2), &xh_map, 0, y, 2 * m + par, &sh->full_tma[s]);
+                        continue;
                     }
 #pragma unroll
                     for (int par = 0; par < 2; ++par)
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
-                            tc::tma_load_3d(st + (par * 2 + 0) * (SB / 8) + h * (SB / 16), &xh_map, h * 64, y,
+                            tc::tma_load_3d(st + (par * 2 + 0) * BL + h * (BL / 2), &xh_map, h * 64, y,
                                             2 * m + par, &sh->full_tma[s]);
-                            tc::tma_load_3d(st + (par * 2 + 1) * (SB / 8) + h * (SB / 16), &xl_map, h * 64, y,
+                            tc::tma_load_3d(st + (par * 2 + 1) * BL + h * (BL / 2), &xl_map, h * 64, y,
                                             2 * m + par, &sh->full_tma[s]);
                         }
                 }
@@ -541,7 +563,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (lane == 0) {
             TCP_DECL;
             TCP_T0(role);
-            const uint32_t idesc = F16 ? tc::idesc_f16(128, kTcCols, true, true) : tc::idesc_bf16(128, kTcCols, true, true);
+            constexpr int N = PK ? 2 * kPkCols : kTcCols;
+            const uint32_t idesc = F16 ? tc::idesc_f16(128, N, true, true) : tc::idesc_bf16(128, N, true, true);
             int it = 0, tcount = 0;
             for (int t = t_begin; t < t_end; ++t, ++tcount) {
                 const int m = tiles[t].x, c0 = fwd_tile_c0(tiles[t].y);
@@ -561,22 +584,28 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     TCP_ADD(0, 1, w1);
                     tc::tc_fence_after();
                     const uint32_t sa = tc::smem_u32(stages + s * SB);
-                    const uint32_t sb = sa + SB / 2;
+                    const uint32_t sb = sa + SA;
 #pragma unroll
                     for (int par = 0; par < 2; ++par) {
-                        const uint32_t dm = tmem + par * 2 * kTcCols, dc = dm + kTcCols;
+                        const uint32_t dm = tmem + par * (PK ? kPkTmem : 2 * kTcCols), dc = dm + NC;
 #pragma unroll
                         for (int ks = 0; ks < RS / 16; ++ks) {
                             // K-step ks: rings 16 ks .. +15, 16 rows of 128 B into each 64-wide half
                             const uint32_t ko = ks * 2048;
-                            const uint64_t ah = tc::smem_desc_sw128(sa + (par * 2 + 0) * (SB / 8) + ko, SB / 16, 1024);
-                            const uint64_t al = tc::smem_desc_sw128(sa + (par * 2 + 1) * (SB / 8) + ko, SB / 16, 1024);
-                            const uint64_t bh = tc::smem_desc_sw128(sb + (par * 2 + 0) * (SB / 8) + ko, SB / 16, 1024);
-                            const uint64_t bl = tc::smem_desc_sw128(sb + (par * 2 + 1) * (SB / 8) + ko, SB / 16, 1024);
+                            const uint64_t ah = tc::smem_desc_sw128(sa + (par * 2 + 0) * BL + ko, BL / 2, 1024);
+                            const uint64_t al = tc::smem_desc_sw128(sa + (par * 2 + 1) * BL + ko, BL / 2, 1024);
                             const uint32_t acc = (c > c0 || ks > 0) ? 1u : 0u;
-                            tc::mma_bf16(dm, ah, bh, idesc, acc);
-                            tc::mma_bf16(dc, ah, bl, idesc, acc);
-                            tc::mma_bf16(dc, al, bh, idesc, 1u);
+                            if constexpr (PK) {
+                                const uint64_t bb = tc::smem_desc_sw128(sb + par * (BL / 2) + ko, BL / 2, 1024);
+                                tc::mma_bf16(dm, ah, bb, idesc, acc);
+                                tc::mma_bf16(dc, al, bb, idesc, 1u);
+                            } else {
+                                const uint64_t bh = tc::smem_desc_sw128(sb + (par * 2 + 0) * BL + ko, BL / 2, 1024);
+                                const uint64_t bl = tc::smem_desc_sw128(sb + (par * 2 + 1) * BL + ko, BL / 2, 1024);
+                                tc::mma_bf16(dm, ah, bh, idesc, acc);
+                                tc::mma_bf16(dc, ah, bl, idesc, acc);
+                                tc::mma_bf16(dc, al, bh, idesc, 1u);
+                            }
                         }
                     }
                     tc::mma_commit(&sh->empty[s]);
@@ -610,12 +639,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll 1
             for (int par = par_lo; par < par_hi; ++par) {
                 const int l = l0 + 2 * row + par;
-                const uint32_t taddr = tmem + ((uint32_t)(ew * 32) << 16) + par * 2 * kTcCols;
+                const uint32_t taddr = tmem + ((uint32_t)(ew * 32) << 16) + par * (PK ? kPkTmem : 2 * kTcCols);
 #pragma unroll 1
-                for (int c = 0; c < kTcCols; c += 16) {
+                for (int c = 0; c < NC; c += 16) {
                     float v[16], w[16];
                     tc::tmem_ld16(taddr + c, v);
-                    tc::tmem_ld16(taddr + kTcCols + c, w);
+                    tc::tmem_ld16(taddr + NC + c, w);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] += w[j];
                     if constexpr (TAB) {
@@ -629,8 +658,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         const int lr0 = l0 + 2 * ew * 32 + par;  // degree of row 0 of this warp
                         epi_store_block(stg, v, lane, [&](int r) -> float* {
                             const int lr = lr0 + 2 * r;
-                            return (lr < L && HPX_INB(((int64_t)m * L + lr) * kTcCols + c + 15, kExtYcols, 13))
-                                       ? ycols + ((int64_t)m * L + lr) * kTcCols + c
+                            return (lr < L && HPX_INB(((int64_t)m * L + lr) * NC + c + 15, kExtYcols, 13))
+                                       ? ycols + ((int64_t)m * L + lr) * NC + c
                                        : nullptr;
                         });
                     } else if (l < L && HPX_INB(((int64_t)m * L + l) * kTcCols + c + 15, kExtYcols, 13)) {
@@ -783,7 +812,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // Chunk it goes to producer pair g = it mod 3 (warps 8+2g, 9+2g), which owns
 // stage g (one barrier phase of run-ahead at most); lane runs rings 32w + lane
 // and 64 + 32w + lane of the tile.
-template <bool F16, bool TAB>
+template <bool F16, bool TAB, bool PK>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_leg_inv_tc(const __grid_constant__ CUtensorMap ah_map, const __grid_constant__ CUtensorMap al_map,
                  const __grid_constant__ CUtensorMap tab_map, const __grid_constant__ CUtensorMap spec_map,
@@ -792,6 +821,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                  const double2* __restrict__ pstart, const double2* __restrict__ coef,
                  const AlphaC* __restrict__ alphac, const double2* __restrict__ seeds, const int2* __restrict__ tiles,
                  const int* __restrict__ tile_off, const unsigned* __restrict__ amax, int* __restrict__ err) {
+    static_assert(TAB || !PK, "packed operands go with the resident table");
+    constexpr int NS = PK ? kPkStages : kIStages, SB = PK ? kPkStageBytes : kIStageBytes, NC = kTcN<PK>;
     __shared__ float s_inv[kTcCols / 2];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // align by pointer arithmetic on the shared array (keeps the shared address space known)
@@ -805,7 +836,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int nbk = seed_blocks(L);
     const int t_begin = tile_off[blockIdx.x], t_end = tile_off[blockIdx.x + 1];  // this CTA's tiles
     load_inv_scales<F16>(s_inv, amax, 1.f, nmaps);
-    tc_setup(sh, kIStages, 2, warp, kEpiWarps<TAB>);
+    tc_setup(sh, NS, 2, warp, kEpiWarps<TAB>);
     const uint32_t tmem = sh->tmem_base;
     auto nchunks = [&](int m) { return m < L ? (L - m + kTcDegChunk - 1) / kTcDegChunk : 0; };
 
@@ -820,17 +851,23 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 const int t0 = geo.first_ring(m);
                 const int nch = nchunks(m);
                 for (int c = c0; c < nch; ++c, ++it) {
-                    const int s = it % kIStages;
-                    if (!tc::mbar_wait(&sh->empty[s], ((it / kIStages) & 1) ^ 1, err, 21)) goto tma_done;
-                    unsigned char* st = stages + s * kIStageBytes + 32768;
-                    tc::mbar_arrive_tx(&sh->full_tma[s], TAB ? 65536 : 32768);
+                    const int s = it % NS;
+                    if (!tc::mbar_wait(&sh->empty[s], ((it / NS) & 1) ^ 1, err, 21)) goto tma_done;
+                    unsigned char* st = stages + s * SB + 32768;
+                    tc::mbar_arrive_tx(&sh->full_tma[s], TAB ? SB : 32768);
                     if (kWithholdTmaLoads) continue;
                     if (TAB) {
                         // A operand: Pbar^T for 128 rings x 32 degrees of each parity, hi and lo
 #pragma unroll
                         for (int ph = 0; ph < 4; ++ph)
-                            tc::tma_load_3d(stages + s * kIStageBytes + ph * 8192, &tab_map, c * (kTcDegChunk / 2),
+                            tc::tma_load_3d(stages + s * SB + ph * 8192, &tab_map, c * (kTcDegChunk / 2),
                                             t0 + rb, 4 * m + ph, &sh->full_tma[s]);
+                    }
+                    if constexpr (PK) {
+#pragma unroll
+                        for (int par = 0; par < 2; ++par)
+                            tc::tma_load_3d(st + par * 4096, &ah_map, 0, c * 32, 2 * m + par, &sh->full_tma[s]);
+                        continue;
                     }
 #pragma unroll
                     for (int par = 0; par < 2; ++par)
@@ -844,13 +881,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
             }
         tma_done:
-            tma_drain(sh, it, kIStages);
+            tma_drain(sh, it, NS);
         }
     } else if (warp == 1) {
         if (lane == 0) {
             TCP_DECL;
             TCP_T0(role);
-            const uint32_t idesc = F16 ? tc::idesc_f16(128, kTcCols, false, true) : tc::idesc_bf16(128, kTcCols, false, true);
+            constexpr int N = PK ? 2 * kPkCols : kTcCols;
+            const uint32_t idesc = F16 ? tc::idesc_f16(128, N, false, true) : tc::idesc_bf16(128, N, false, true);
             int it = 0, tcount = 0;
             for (int t = t_begin; t < t_end; ++t, ++tcount) {
                 const int m = tiles[t].x, c0 = inv_tile_c0(tiles[t].y);
@@ -860,8 +898,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 TCP_ADD(1, 2, w2);
                 tc::tc_fence_after();
                 for (int c = c0; c < nch; ++c, ++it) {
-                    const int s = it % kIStages;
-                    const uint32_t ph = (it / kIStages) & 1;
+                    const int s = it % NS;
+                    const uint32_t ph = (it / NS) & 1;
                     TCP_T0(w0);
                     if (!tc::mbar_wait(&sh->full_tma[s], ph, err, 23)) goto mma_done;
                     TCP_ADD(1, 0, w0);
@@ -869,21 +907,27 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     if (!TAB && !tc::mbar_wait(&sh->full_prod[s], ph, err, 24)) goto mma_done;
                     TCP_ADD(1, 1, w1);
                     tc::tc_fence_after();
-                    const uint32_t sa = tc::smem_u32(stages + s * kIStageBytes);
+                    const uint32_t sa = tc::smem_u32(stages + s * SB);
                     const uint32_t sb = sa + 32768;
 #pragma unroll
                     for (int par = 0; par < 2; ++par) {
-                        const uint32_t dm = tmem + par * 2 * kTcCols, dc = dm + kTcCols;
+                        const uint32_t dm = tmem + par * (PK ? kPkTmem : 2 * kTcCols), dc = dm + NC;
 #pragma unroll
                         for (int ks = 0; ks < 2; ++ks) {
                             const uint64_t ah = tc::smem_desc_kmajor_sw64(sa + (par * 2 + 0) * 8192 + ks * 32, 512);
                             const uint64_t al = tc::smem_desc_kmajor_sw64(sa + (par * 2 + 1) * 8192 + ks * 32, 512);
-                            const uint64_t bh = tc::smem_desc_sw128(sb + (par * 2 + 0) * 8192 + ks * 2048, 4096, 1024);
-                            const uint64_t bl = tc::smem_desc_sw128(sb + (par * 2 + 1) * 8192 + ks * 2048, 4096, 1024);
                             const uint32_t acc = (c > c0 || ks > 0) ? 1u : 0u;
-                            tc::mma_bf16(dm, ah, bh, idesc, acc);
-                            tc::mma_bf16(dc, ah, bl, idesc, acc);
-                            tc::mma_bf16(dc, al, bh, idesc, 1u);
+                            if constexpr (PK) {
+                                const uint64_t bb = tc::smem_desc_sw128(sb + par * 4096 + ks * 2048, 4096, 1024);
+                                tc::mma_bf16(dm, ah, bb, idesc, acc);
+                                tc::mma_bf16(dc, al, bb, idesc, 1u);
+                            } else {
+                                const uint64_t bh = tc::smem_desc_sw128(sb + (par * 2 + 0) * 8192 + ks * 2048, 4096, 1024);
+                                const uint64_t bl = tc::smem_desc_sw128(sb + (par * 2 + 1) * 8192 + ks * 2048, 4096, 1024);
+                                tc::mma_bf16(dm, ah, bh, idesc, acc);
+                                tc::mma_bf16(dc, ah, bl, idesc, acc);
+                                tc::mma_bf16(dc, al, bh, idesc, 1u);
+                            }
                         }
                     }
                     tc::mma_commit(&sh->empty[s]);
@@ -915,12 +959,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll 1
             for (int par = par_lo; par < par_hi; ++par) {
                 float* dst = spec + (((int64_t)m * 2 + par) * NP + p) * C;
-                const uint32_t taddr = tmem + ((uint32_t)(ew * 32) << 16) + par * 2 * kTcCols;
+                const uint32_t taddr = tmem + ((uint32_t)(ew * 32) << 16) + par * (PK ? kPkTmem : 2 * kTcCols);
 #pragma unroll 1
-                for (int c = 0; c < kTcCols; c += 16) {
+                for (int c = 0; c < NC; c += 16) {
                     float v[16], w[16];
                     tc::tmem_ld16(taddr + c, v);
-                    tc::tmem_ld16(taddr + kTcCols + c, w);
+                    tc::tmem_ld16(taddr + NC + c, w);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] += w[j];
                     if constexpr (TAB) {
@@ -1086,38 +1130,41 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // degree l = m + 2i + par; rows with l >= L (up to L+63) are written as zeros.
 // amax != nullptr: fp16 halves of the values times 2^e(map), e from the map's
 // max |a| (k_alm_maxabs); otherwise bf16 halves.
+template <int NB>
 __global__ void k_alm_to_tc(const float* __restrict__ alm, int nmaps, int L, int M, int Lh,
                             uint16_t* __restrict__ ah, uint16_t* __restrict__ al, const unsigned* __restrict__ amax) {
-    __shared__ float2 tile[64][33];
-    __shared__ float s_sc[64];
+    // NB = 64: rows of 128 columns in two planes; kPkMaps: packed rows of [hi 32 | lo 32]
+    constexpr int RW = NB == 64 ? kTcCols : 2 * kPkCols;
+    __shared__ float2 tile[NB][33];
+    __shared__ float s_sc[NB];
     const int m0 = blockIdx.x * 32, l = blockIdx.y;
     if (l < m0) return;  // only m <= l is used: nothing to convert in this block
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
     // all loads of the thread are issued before the first shared-memory store
-    float2 vv[8];
+    float2 vv[NB / 8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < NB / 8; ++k) {
         const int i = ty + 8 * k, m = m0 + tx;
         vv[k] = make_float2(0.f, 0.f);
         if (i < nmaps && m < M && m <= l && l < L && HPX_INB(2 * (((int64_t)i * L + l) * M + m) + 1, kExtAlm, 9))
             vv[k] = *(const float2*)(alm + 2 * (((int64_t)i * L + l) * M + m));
     }
-    if (amax && ty < 2) {
+    if (amax && ty * 32 + tx < NB) {
         const int b = ty * 32 + tx;
         s_sc[b] = tc::pow2f(tc::f16_scale_exp(__uint_as_float(b < nmaps ? amax[b] : 0u)));
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) tile[ty + 8 * k][tx] = vv[k];
+    for (int k = 0; k < NB / 8; ++k) tile[ty + 8 * k][tx] = vv[k];
     __syncthreads();
     // each warp writes rows for 4 m's: 128 columns as 64 bf16x2 (hi) + 64 (lo)
     for (int mi = ty; mi < 32; mi += 8) {
         const int m = m0 + mi;
         if (m >= M || l < m) continue;
         const int d = l - m, par = d & 1, i = d >> 1;
-        if (i >= Lh || !HPX_INB((((int64_t)(2 * m + par)) * Lh + i) * kTcCols + kTcCols - 1, kExtOperA, 10)) continue;
-        uint32_t* rh = (uint32_t*)(ah + (((int64_t)(2 * m + par)) * Lh + i) * kTcCols);
-        uint32_t* rl = (uint32_t*)(al + (((int64_t)(2 * m + par)) * Lh + i) * kTcCols);
-        for (int b = tx; b < 64; b += 32) {
+        if (i >= Lh || !HPX_INB((((int64_t)(2 * m + par)) * Lh + i) * RW + RW - 1, kExtOperA, 10)) continue;
+        uint32_t* rh = (uint32_t*)(ah + (((int64_t)(2 * m + par)) * Lh + i) * RW);
+        uint32_t* rl = (uint32_t*)(al + (((int64_t)(2 * m + par)) * Lh + i) * RW);
+        for (int b = tx; b < NB; b += 32) {
             const float2 v = tile[b][mi];
             uint16_t h0, l0, h1, l1;
             if (amax) {
@@ -1139,29 +1186,27 @@ __global__ void k_alm_to_tc(const float* __restrict__ alm, int nmaps, int L, int
 // l < m entries are set to zero unless accumulating.  Grid (ceil(m_end/32), L),
 // block 32 x 8; the transpose goes through shared memory so that both the
 // 512-byte row reads and the 32-order stores are coalesced.
+template <int NB>
 __global__ void k_tc_to_alm(const float* __restrict__ ycols, int nmaps, int L, int M, int m_end,
                             float* __restrict__ alm, int accumulate) {
-    __shared__ float2 tile[64][33];
+    __shared__ float2 tile[NB][33];
     const int m0 = blockIdx.x * 32, l = blockIdx.y;
-    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+    constexpr int NL = 32 * NB / 256;
     // all loads of the thread are issued before the first shared-memory store
-    float2 vv[4][2];
+    float2 vv[NL];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int m = m0 + ty + 8 * k;
-        const bool live = m < m_end && m <= l && HPX_INB(((int64_t)m * L + l) * kTcCols + kTcCols - 1, kExtYcols, 11);
-        const float2* row = (const float2*)(ycols + ((int64_t)m * L + l) * kTcCols);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) vv[k][h] = live ? row[tx + 32 * h] : make_float2(0.f, 0.f);
+    for (int k = 0; k < NL; ++k) {
+        const int i = tid + 256 * k, m = m0 + i / NB;
+        const bool live = m < m_end && m <= l && HPX_INB(((int64_t)m * L + l) * 2 * NB + 2 * NB - 1, kExtYcols, 11);
+        vv[k] = live ? ((const float2*)(ycols + ((int64_t)m * L + l) * 2 * NB))[i % NB] : make_float2(0.f, 0.f);
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) tile[tx + 32 * h][ty + 8 * k] = vv[k][h];
+    for (int k = 0; k < NL; ++k) tile[(tid + 256 * k) % NB][(tid + 256 * k) / NB] = vv[k];
     __syncthreads();
     const int m = m0 + tx;
     if (m >= m_end) return;
-    for (int b = ty; b < nmaps && b < 64; b += 8) {
+    for (int b = ty; b < nmaps && b < NB; b += 8) {
         if (!HPX_INB(2 * (((int64_t)b * L + l) * M + m) + 1, kExtAlm, 12)) continue;
         float2* dst = (float2*)(alm + 2 * (((int64_t)b * L + l) * M + m));
         float2 v = tile[b][tx];
