@@ -1234,8 +1234,24 @@ struct Pipeline {
     // (legendre_direct.cuh): FP32 wherever the tiled ones are not the better,
     // FP64 synthesis always (nside 256, 32 maps: 957 us against 2583 us of the tiled
     // kernel it replaced) and FP64 analysis up to 30 maps (nside 256: 16 maps 1107
-    // us against 1793 tiled, 32 maps 2003 against 1977).
-    bool direct_fwd(int nb) const { return !P->mixed() && (sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 30); }
+    // us against 1793 tiled, 32 maps 2003 against 1977); and the FP32 ones in mixed
+    // plans for a few maps, which pay the tensor-core kernels' whole table
+    // stream and layout passes (and come out more accurate): whole calls,
+    // direct / tensor cores, nside 1024 analysis 2 maps 2.3 / 2.8 ms, 4 maps 3.6 /
+    // 2.9, synthesis 4 maps 2.7 / 3.0, 8 maps 4.8 / 3.3; nside 256 analysis 4 maps
+    // 125 / 135 us, 8 maps 222 / 152, synthesis 8 maps 145 / 163, 12 maps 212 / 183;
+    // nside 64 16 maps 39 / 40 and 33 / 46.  Plans without the table
+    // generate Pbar either way and cross over later.
+    bool direct_fwd(int nb) const {
+        if (P->mixed()) return nb <= mixed_direct(2, 4, 8);
+        return sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 30;
+    }
+    bool direct_inv(int nb) const { return P->mixed() ? nb <= mixed_direct(4, 8, 12) : !tile_inv(nb); }
+    int mixed_direct(int large, int medium, int no_table) const {
+        if (kWithholdTmaLoads) return 0;  // the failure-detection build keeps to the pipeline it tests
+        if (!P->tc.table) return no_table;
+        return P->NP <= 128 ? 16 : P->NP <= 512 ? medium : large;
+    }
     const typename DirRec<T>::Coef* dir_coef() const {
         if constexpr (sizeof(T) == 4) return P->d_alpha;
         else return P->d_coef;
@@ -1357,14 +1373,14 @@ struct Pipeline {
     bool tile_inv(int nb) const { return P->tiled() && P->NP >= 256 && nb > (P->NP >= 512 ? 46 : 56); }
     // alm -> map (ref: residual ref - map)
     void synthesis(const T* alm, T* map, int nb, int adjoint, const T* ref) {
-        if (tile_inv(nb)) {
-            if constexpr (sizeof(T) == 4) leg_inv_tile(alm, nb);
-            ring_inv(map, nb, adjoint, ref);
-        } else if (!P->mixed()) {
+        if (direct_inv(nb)) {
             leg_inv_direct(alm, nb, adjoint);
             ring_fft_inv(map, nb, ref);
-        } else {
-            leg_inv(alm, nb);
+            return;
+        }
+        if constexpr (sizeof(T) == 4) {
+            if (P->mixed()) leg_inv(alm, nb);
+            else leg_inv_tile(alm, nb);
             ring_inv(map, nb, adjoint, ref);
         }
     }

@@ -90,3 +90,21 @@ def test_direct_spin1_against_oracle(cuda, nside, L, M, batch, dtype):
     assert rel(a, ref) < tol
     y = hpx.VectoriSHTCUDA(nside, L, M)(torch.from_numpy(ref).to(cuda, a.dtype))
     assert rel(y, V.visht(ref, nside)) < tol
+
+
+# mixed plans: a few maps take the FP32 direct contractions (with and without the
+# Legendre table), one more takes the tensor cores
+@pytest.mark.parametrize("nside,L,M,few,table", [(32, 65, 63, 16, True), (128, 200, 150, 4, True), (32, 65, 63, 8, False)])
+def test_mixed_plans_of_few_maps(cuda, nside, L, M, few, table):
+    import cuhpx_b200 as hpx
+
+    rng = np.random.default_rng(nside)
+    f = rng.standard_normal((few + 1, 12 * nside * nside))
+    ref = O.sht(f[:2], nside, L, M)
+    x = torch.from_numpy(f).float().to(cuda)
+    kw = dict(lmax=L, mmax=M, precision="f16x3", legendre_table=table)
+    for n in (2, few, few + 1):
+        a = hpx.SHTCUDA(nside, **kw)(x[:n])
+        assert rel(a[:2], ref) < 2e-6
+        y = hpx.iSHTCUDA(nside, **kw)(a)
+        assert rel(y[:2], O.isht(ref, nside)) < 4e-6
