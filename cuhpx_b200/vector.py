@@ -12,8 +12,6 @@ order than the transform, which the derivative table needs.  Gradients are
 the exact adjoints (the reference differentiates its einsums by autograd).
 """
 
-import ctypes
-
 import torch
 import torch.nn as nn
 
@@ -21,28 +19,18 @@ from . import _lib
 from .hpx_sht import get_plan
 
 
-def _call(fn, plan, src, dst, batch, csphase):
-    ws, nbytes = plan._ws(batch, src.device)
-    stream = torch.cuda.current_stream(src.device).cuda_stream
-    _lib.check(fn(plan._h, ctypes.c_void_p(src.data_ptr()), ctypes.c_void_p(dst.data_ptr()), int(batch),
-                  int(csphase), ctypes.c_void_p(ws.data_ptr()), nbytes, ctypes.c_void_p(stream)), plan._h)
-    return dst
-
-
 def _analysis(plan, x, L, M, csphase, adjoint=False):
     B = x.shape[0]
     out = torch.empty((B, 2, L, M), dtype=plan.cdtype, device=x.device)
     fn = plan._lib.hpx_vsht_inverse_adjoint if adjoint else plan._lib.hpx_vsht_forward
-    _call(fn, plan, x, torch.view_as_real(out), B, csphase)
-    return out
+    return plan._call(fn, x, out, B, int(csphase))
 
 
 def _synthesis(plan, a, csphase, adjoint=False):
     B = a.shape[0]
     out = torch.empty((B, 2, plan.npix), dtype=plan.dtype, device=a.device)
     fn = plan._lib.hpx_vsht_forward_adjoint if adjoint else plan._lib.hpx_vsht_inverse
-    _call(fn, plan, torch.view_as_real(a.resolve_conj().contiguous()), out, B, csphase)
-    return out
+    return plan._call(fn, a.resolve_conj().contiguous(), out, B, int(csphase))
 
 
 class VectorSHTFunction(torch.autograd.Function):
