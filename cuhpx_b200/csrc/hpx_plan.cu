@@ -1758,8 +1758,9 @@ int dispatch_remap_async(const E* in, E* out, const RemapLaunch& L) {
 
 // Remap launcher: squares of 64 x 64 pixels for elements of up to 4 bytes and
 // 32 x 32 above, fewer for nside < 64.  Map groups of up to 16 maps a CTA
-// amortise the offsets' arithmetic, while leaving at least 16 CTAs a
-// multiprocessor.  Elements of 4, 8 and 16 bytes take the cp.async pipeline
+// amortise the offsets' arithmetic, while leaving at least 8 CTAs a
+// multiprocessor (nside 512, 16 float maps, nest2ring / ring2nest: 8 CTAs 104 / 108
+// us, 16 CTAs 112 / 130, 4 CTAs 108 / 107).  Elements of 4, 8 and 16 bytes take the cp.async pipeline
 // (16-byte accesses on NEST and XY sides when the tiles are at least 16 bytes
 // wide and both buffers 16-byte aligned); 1- and 2-byte elements stage
 // through registers.
@@ -1772,10 +1773,10 @@ int launch_remap(const void* in, void* out, int64_t batch, int nside, RemapSide 
     const int log_tiles = logn - logs;
     const int64_t tiles = 12ll << (2 * log_tiles);
     int mpc = 16;
-    while (mpc > 1 && tiles * ((batch + mpc - 1) / mpc) < 148ll * 16) mpc >>= 1;
+    while (mpc > 1 && tiles * ((batch + mpc - 1) / mpc) < 148ll * 8) mpc >>= 1;
     const bool ring = src.order == kOrderRing || dst.order == kOrderRing;
     constexpr bool kAsync = sizeof(E) >= 4;
-    const size_t smem = kAsync ? remap_async_smem_bytes(s, (int)sizeof(E), ring)
+    const size_t smem = kAsync ? remap_async_smem_bytes(s, (int)sizeof(E), dst.order == kOrderRing)
                                : remap_smem_bytes(s, (int)sizeof(E), ring);
     const int vec = (s * (int)sizeof(E) >= 16 && ((((uintptr_t)in) | ((uintptr_t)out)) & 15) == 0) ? 1 : 0;
     const int64_t np = 12ll * nside * nside;

@@ -99,25 +99,24 @@ HPX_HD void flat_to_xy(int& x, int& y, const RemapSide& s, int mask) {
 // at the north pole; nr: pixels of that ring per base face; jp: 1-based
 // position in the ring (wraps once for the equatorial face 4, whose column
 // starts at phi = 0).
-HPX_HD int64_t xyf_to_ring(int ix, int iy, int f, int nside) {
-    const int64_t n = nside;
-    const int64_t jr = (int64_t)((f >> 2) + 2) * n - ix - iy - 1;
-    int64_t nr, before;
-    int kshift = 0;
+// 32-bit throughout: hpx_remap takes nside up to 8192 (12 nside^2 < 2^30).
+HPX_HD int xyf_to_ring(int ix, int iy, int f, int n) {
+    const int jr = ((f >> 2) + 2) * n - ix - iy - 1;
+    int nr, before, kshift = 0;
     if (jr < n) {  // north polar cap
         nr = jr;
         before = 2 * jr * (jr - 1);
     } else if (jr < 3 * n) {  // equatorial belt (rings alternate their shift)
         nr = n;
         before = 2 * n * (n - 1) + (jr - n) * 4 * n;
-        kshift = (int)((jr - n) & 1);
+        kshift = (jr - n) & 1;
     } else {  // south polar cap
-        const int64_t js = 4 * n - jr;
+        const int js = 4 * n - jr;
         nr = js;
         before = 12 * n * n - 2 * js * (js + 1);
     }
     const int jpll = ((f & 3) << 1) - ((f >> 2) & 1) + 1;  // face column, in half faces
-    int64_t jp = (jpll * nr + ix - iy + 1 + kshift) / 2;  // numerator is even
+    int jp = (jpll * nr + ix - iy + 1 + kshift) / 2;  // numerator is even
     if (jp < 1) jp += 4 * n;
     return before + jp - 1;
 }
@@ -325,21 +324,27 @@ __global__ void __launch_bounds__(kRemapThreads, 5) k_remap(const E* __restrict_
 // hold them) and one barrier per map ordering the ring.  NEST and XY sides
 // move V = 16 / sizeof(E) consecutive pixels per access (one 16-byte cp.async
 // or store: a NEST tile is one run, an XY tile s rows of s >= V); a RING side
-// moves single elements along its diagonal runs, whose offsets come from the
-// tile's table.  Shared-memory tiles are unpadded: the V-element vectors of
+// moves single elements along its diagonal runs, whose offsets (and staged slots)
+// each thread keeps in registers for all maps of the CTA instead of reading
+// them from shared tables per map: at nside 1024, 32 float maps, ring2nest 871 -> 695
+// us, ring2flat 905 -> 721, flat2ring 870 -> 847; nest2ring stays at 3.7 TB/s, held by
+// its one-element stores.  Shared-memory tiles are unpadded: the V-element vectors of
 // each 32-element row are XOR-swizzled by the row number, which keeps every
 // vector 16-byte aligned while spreading transposed and diagonal reads over
-// the banks.  64 x 64 float tiles: 72 KB per CTA, three CTAs and six maps of
-// loads (96 KB) in flight per SM.
+// the banks.  64 x 64 float tiles: 48 to 56 KB per CTA, three CTAs and six maps
+// of loads (96 KB) in flight per SM.
 constexpr int kRemapStages = 3;
 
 template <int V>
 HPX_HD int remap_swz(int p) {
     return p ^ (((p >> 5) & (32 / V - 1)) * V);
 }
-HPX_HD size_t remap_async_smem_bytes(int s, int elem, bool ring) {
-    return kRemapStages * (((size_t)s * s * elem + 15) & ~(size_t)15) + remap_slot_bytes(s) +
-           (ring ? (size_t)s * s * 4 : 0);
+// largest tile over the threads: 64 x 64 pixels of 4 bytes, 32 x 32 of 8 and 16
+template <int BYTES>
+constexpr int remap_pixels_per_thread() { return ((BYTES <= 4 ? 64 * 64 : 32 * 32) + kRemapThreads - 1) / kRemapThreads; }
+// staged tiles, and the slot table unless a RING destination keeps it in registers
+HPX_HD size_t remap_async_smem_bytes(int s, int elem, bool ring_dst) {
+    return kRemapStages * (((size_t)s * s * elem + 15) & ~(size_t)15) + (ring_dst ? 0 : remap_slot_bytes(s));
 }
 
 template <int BYTES>
@@ -371,7 +376,15 @@ __global__ void __launch_bounds__(kRemapThreads) k_remap_async(const E* __restri
     const int s = 1 << logs, ss = s * s;
     const size_t tb = ((size_t)ss * sizeof(E) + 15) & ~(size_t)15;
     uint16_t* sslot = reinterpret_cast<uint16_t*>(remap_smem + kRemapStages * tb);
-    uint32_t* ring_tab = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(sslot) + remap_slot_bytes(s));
+    // a thread's pixels on a RING side: offsets (and, for a RING destination, the
+    // staged slots they read) stay in registers for all maps of the CTA
+    constexpr int R = remap_pixels_per_thread<sizeof(E)>();
+    uint32_t roff[R], rslot[R];
+    // RING side: the tables are formed (by a rolled loop: the index arithmetic
+    // unrolled over a thread's pixels cost more in instruction fetches than the
+    // registers saved) in the stages, before the first copy is issued
+    uint32_t* ring_tab = reinterpret_cast<uint32_t*>(remap_smem);
+    uint16_t* ring_slot = reinterpret_cast<uint16_t*>(ring_tab + ss);
 
     // tile, bases and tables (the slot table holds swizzled source positions)
     Tile t;
@@ -395,8 +408,22 @@ __global__ void __launch_bounds__(kRemapThreads) k_remap_async(const E* __restri
             ring_tab[p] = side_offset(t, src, lx, ly);
         }
         side_coords(t, dst, dfx, dfy, p, lx, ly);
-        if constexpr (DO == kOrderRing) ring_tab[p] = side_offset(t, dst, lx, ly);
-        sslot[p] = (uint16_t)remap_swz<V>(side_pos(t, src, sfx, sfy, lx, ly));
+        const int slot = remap_swz<V>(side_pos(t, src, sfx, sfy, lx, ly));
+        if constexpr (DO == kOrderRing) {
+            ring_tab[p] = side_offset(t, dst, lx, ly);
+            ring_slot[p] = (uint16_t)slot;
+        } else {
+            sslot[p] = (uint16_t)slot;
+        }
+    }
+    // (a thread reads back the entries it wrote)
+    if constexpr (SO == kOrderRing || DO == kOrderRing) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int p = threadIdx.x + r * kRemapThreads;
+            roff[r] = p < ss ? ring_tab[p] : 0;
+            rslot[r] = DO == kOrderRing && p < ss ? ring_slot[p] : 0;
+        }
     }
     __syncthreads();
 
@@ -406,8 +433,11 @@ __global__ void __launch_bounds__(kRemapThreads) k_remap_async(const E* __restri
         E* tl = reinterpret_cast<E*>(remap_smem + ((b - b0) % kRemapStages) * tb);
         const E* ib = in + (int64_t)b * npix;
         if constexpr (SO == kOrderRing) {
-            for (int p = threadIdx.x; p < ss; p += kRemapThreads)
-                cp_async_elem<sizeof(E)>(tl + remap_swz<V>(p), ib + ring_tab[p]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int p = threadIdx.x + r * kRemapThreads;
+                if (p < ss) cp_async_elem<sizeof(E)>(tl + remap_swz<V>(p), ib + roff[r]);
+            }
         } else if (vec) {
             for (int p = threadIdx.x * V; p < ss; p += kRemapThreads * V)
                 cp_async16(tl + remap_swz<V>(p), ib + nat_offset<SO>(sbase, p, logs, nside));
@@ -431,7 +461,9 @@ __global__ void __launch_bounds__(kRemapThreads) k_remap_async(const E* __restri
         const E* tl = reinterpret_cast<const E*>(remap_smem + ((b - b0) % kRemapStages) * tb);
         E* ob = out + (int64_t)b * npix;
         if constexpr (DO == kOrderRing) {
-            for (int p = threadIdx.x; p < ss; p += kRemapThreads) ob[ring_tab[p]] = tl[sslot[p]];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if ((int)threadIdx.x + r * kRemapThreads < ss) ob[roff[r]] = tl[rslot[r]];
         } else if (vec) {
             for (int p = threadIdx.x * V; p < ss; p += kRemapThreads * V) {
                 union {
