@@ -319,16 +319,16 @@ __global__ void __launch_bounds__(256) k_alm_maxabs(const float* __restrict__ al
 // Output spec[m][par][p][col] in T, or hi/lo pairs xh/xl (mixed plans): bf16,
 // or, with fmax given, fp16 of the values times 2^e(map), e from the map's
 // max |F| (recorded by k_ring_fwd) times the bound wb on |c| (F_t + F_t').
-// Rows are C wide, of which ncols are columns (hi and lo packed into one row: C = 2
-// ncols, xl = xh + ncols / 2).  CTA per (block of orders, ring pair, NB = 64 or 16
-// maps); the transpose goes through shared memory.
+// Rows are C wide; NB = 16 packs the hi and lo halves of its 32 columns into one
+// (C = 64, xl = xh + 16).  CTA per (block of orders, ring pair, NB = 64 or 16 maps);
+// the transpose goes through shared memory.
 template <typename T, int NB>
 constexpr int fold_mb() { return (sizeof(T) == 4 ? 2048 : 1024) / NB; }
 
 template <typename T, int NB>
 __global__ void __launch_bounds__(256) k_fold(const T* __restrict__ F, int64_t Ftot, int nmaps, Geom geo,
                                               const RingPair* __restrict__ pairs, int adjoint, T* __restrict__ spec,
-                                              int C, int ncols, uint32_t* __restrict__ xh, uint32_t* __restrict__ xl,
+                                              int C, uint32_t* __restrict__ xh, uint32_t* __restrict__ xl,
                                               const unsigned* __restrict__ fmax, float wb) {
     constexpr int MB = fold_mb<T, NB>();
     constexpr int NL = NB * MB / 256;  // elements per thread (the kernel runs 256 threads)
@@ -371,8 +371,8 @@ __global__ void __launch_bounds__(256) k_fold(const T* __restrict__ F, int64_t F
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const int i = tid + 256 * k;
-        const int mm = i / NB, bl = i % NB, b = bz + bl, m = m0 + mm;
-        if (m >= rp.mt || 2 * b >= ncols) continue;
+        const int mm = (unsigned)i / NB, bl = i & (NB - 1), b = bz + bl, m = m0 + mm;
+        if (m >= rp.mt || 2 * b >= (NB == 64 ? C : NB * 2)) continue;
         const T wk = adjoint ? ((m == 0 || m == rp.h) ? (T)1 : (T)2) : (T)rp.w;
         const cplx<T> a = tn[bl][mm], c = ts[bl][mm];
         cplx<T> S, D;
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(256) k_unfold(const T* __restrict__ spec, int 
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const int i = tid + 256 * k;
-        const int mm = i / NB, bl = i % NB, b = bz + bl, m = m0 + mm;
+        const int mm = (unsigned)i / NB, bl = i & (NB - 1), b = bz + bl, m = m0 + mm;
         ve[k] = {(T)0, (T)0};
         vo[k] = {(T)0, (T)0};
         if (m < rp.mt && 2 * b < C && HPX_INB((((int64_t)m * 2 + 1) * NP + p) * C + 2 * b + 1, kExtSpec, 7)) {
@@ -448,8 +448,8 @@ __global__ void __launch_bounds__(256) k_unfold(const T* __restrict__ spec, int 
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const int i = tid + 256 * k;
-        te[i / NB][i % NB] = ve[k];
-        to[i / NB][i % NB] = vo[k];
+        te[(unsigned)i / NB][i & (NB - 1)] = ve[k];
+        to[(unsigned)i / NB][i & (NB - 1)] = vo[k];
     }
     __syncthreads();
 #pragma unroll

@@ -1181,12 +1181,12 @@ struct Pipeline {
         if (packed(nb)) {
             if constexpr (sizeof(T) == 4)
                 k_fold<T, kPkMaps><<<fold_grid<kPkMaps>(nb), 256, 0, st>>>(F, P->Ftot, nb, P->geo, P->d_pairs, adjoint, spec,
-                                                                          2 * kPkCols, kPkCols, xh(), xh() + kPkCols / 2,
-                                                                          fmax, fold_wb);
+                                                                          2 * kPkCols, xh(), xh() + kPkCols / 2, fmax,
+                                                                          fold_wb);
             return;
         }
         k_fold<T, 64><<<fold_grid<64>(nb), 256, 0, st>>>(F, P->Ftot, nb, P->geo, P->d_pairs, adjoint, spec, P->cols(),
-                                                        P->cols(), xh(), xl(), fmax, fold_wb);
+                                                        xh(), xl(), fmax, fold_wb);
     }
     // synthesis output spec (E/O) -> ring spectra F -> map (ref: residual ref - map)
     void ring_inv(T* map, int nb, int adjoint, const T* ref) {
