@@ -248,8 +248,10 @@ constexpr int max_degrees() { return sizeof(T) == 4 ? 12956 : 11420; }
 // dynamic shared memory limits of the direct kernels (per function, as above)
 template <typename T, int C, int R>
 cudaError_t direct_attribute(int bytes) {
-    cudaError_t e = cudaFuncSetAttribute(k_leg_fwd_direct<T, C, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
+    if constexpr (sizeof(T) == 4 || C < 8) {
+        cudaError_t e = cudaFuncSetAttribute(k_leg_fwd_direct<T, C, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+    }
     return cudaFuncSetAttribute(k_leg_inv_direct<T, C, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes - 1024);
 }
 template <typename T, int CV, int R>
@@ -1233,8 +1235,11 @@ struct Pipeline {
     // The contractions that read and write the ring spectra themselves
     // (legendre_direct.cuh): FP32 wherever the tiled ones are not the better,
     // FP64 synthesis always (nside 256, 32 maps: 957 us against 2583 us of the tiled
-    // kernel it replaced) and FP64 analysis up to 30 maps (nside 256: 16 maps 1107
-    // us against 1793 tiled, 32 maps 2003 against 1977); and the FP32 ones in mixed
+    // kernel it replaced) and FP64 analysis up to 48 maps, beyond which the tiled
+    // kernel's cost for 64 columns spreads over enough of them (whole calls, direct
+    // against tiled, nside 256: 16 maps 771 / 1748 us, 32 maps 1385 / 1903, 48 maps
+    // 1996 / 2074, 56 maps 2321 / 2175; nside 512: 48 maps 12.7 / 13.1 ms, 64 maps
+    // 16.8 / 13.8); and the FP32 ones in mixed
     // plans for a few maps, which pay the tensor-core kernels' whole table
     // stream and layout passes (and come out more accurate): whole calls,
     // direct / tensor cores, nside 1024 analysis 2 maps 2.3 / 2.8 ms, 4 maps 3.6 /
@@ -1244,7 +1249,7 @@ struct Pipeline {
     // generate Pbar either way and cross over later.
     bool direct_fwd(int nb) const {
         if (P->mixed()) return nb <= mixed_direct(2, 4, 8);
-        return sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 30;
+        return sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 48;
     }
     bool direct_inv(int nb) const { return P->mixed() ? nb <= mixed_direct(4, 8, 12) : !tile_inv(nb); }
     int mixed_direct(int large, int medium, int no_table) const {
@@ -1291,11 +1296,17 @@ struct Pipeline {
     // CTAs an SM (nside 128, 8 maps: 30 us against 36).
     void leg_fwd_direct(T* alm, int nb, int adjoint, int accumulate) {
         Timer tm(P, st, kStLegFwd);
-        constexpr int R8 = sizeof(T) == 4 ? 4 : 2;
         const bool small = P->NP <= 64;
-        if (nb == 1) small ? leg_fwd_direct_launch<2, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<2, 4>(alm, nb, adjoint, accumulate);
-        else if (nb == 2) small ? leg_fwd_direct_launch<4, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<4, 4>(alm, nb, adjoint, accumulate);
-        else small ? leg_fwd_direct_launch<8, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<8, R8>(alm, nb, adjoint, accumulate);
+        if (nb == 1) {
+            small ? leg_fwd_direct_launch<2, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<2, 4>(alm, nb, adjoint, accumulate);
+        } else if (nb == 2 || sizeof(T) == 8) {
+            // FP64: two maps at a time leave room for R = 4 (nside 512, 4 maps:
+            // 1069 us against 1490 with four maps and R = 2; nside 128, degrees < 511,
+            // 4 maps: 76 against 88)
+            small ? leg_fwd_direct_launch<4, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<4, 4>(alm, nb, adjoint, accumulate);
+        } else if constexpr (sizeof(T) == 4) {
+            small ? leg_fwd_direct_launch<8, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<8, 4>(alm, nb, adjoint, accumulate);
+        }
     }
     void leg_inv_direct(const T* alm, int nb, int adjoint) {
         Timer tm(P, st, kStLegInv);

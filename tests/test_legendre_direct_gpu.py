@@ -108,3 +108,17 @@ def test_mixed_plans_of_few_maps(cuda, nside, L, M, few, table):
         assert rel(a[:2], ref) < 2e-6
         y = hpx.iSHTCUDA(nside, **kw)(a)
         assert rel(y[:2], O.isht(ref, nside)) < 4e-6
+
+
+@pytest.mark.parametrize("batch", [31, 48, 49, 67])
+def test_fp64_analysis_around_the_tiled_kernel(cuda, batch):
+    """FP64 analysis changes kernels above 48 maps of a block of up to 64."""
+    import cuhpx_b200 as hpx
+
+    nside, L, M = 12, 30, 29
+    f = np.random.default_rng(batch).standard_normal((batch, 12 * nside * nside))
+    ref = O.sht(f, nside, L, M, quad_weights="none")
+    sht = hpx.SHTCUDA(nside, lmax=L, mmax=M, quad_weights="none")
+    a = sht(torch.from_numpy(f).to(cuda))
+    assert rel(a, ref) < 1e-11
+    assert rel(a[batch - 1], ref[batch - 1]) < 1e-11
