@@ -1289,7 +1289,7 @@ struct Pipeline {
     // Columns C: those of the map group, up to 8 (4 maps: beyond that the
     // registers of the column values leave no room for R rings).  Rings R per
     // lane: 4 (FP32 analysis at nside 1024, one map: 1566 us against 1836 with
-    // R = 2; synthesis 1327 against 1731), 2 where the wider FP64 columns would
+    // R = 2, both before sum_perm; synthesis 1327 against 1731), 2 where the wider FP64 columns would
     // spill (C = 8: synthesis 58 us against 78 at nside 128, L = 511, 4 maps)
     // and where R = 4 leaves a small plan too few warps: analysis with one block
     // of 64 ring pairs (nside 32: 10.6 us against 12.4), synthesis below three

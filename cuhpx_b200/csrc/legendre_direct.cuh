@@ -24,8 +24,8 @@
 // operations (15%); what keeps them from more is latency -- 12 to 16 warps an SM fit beside
 // the column values.  Measured against the tiled kernels (64 map columns
 // whatever the batch) they replaced, analysis + synthesis contraction alone: one
-// map at nside 1024, L = M = 2047, FP32 71.3 -> 2.9 ms; 8 maps at nside 256, L
-// = M = 511 1370 -> 275 us; 4 maps at nside 128, L = 511, FP64 1412 -> 150 us.
+// map at nside 1024, L = M = 2047, FP32 71.3 -> 2.85 ms; 8 maps at nside 256, L
+// = M = 511 1370 -> 266 us; 4 maps at nside 128, L = 511, FP64 1412 -> 125 us.
 #pragma once
 
 #include "legendre.cuh"
@@ -167,14 +167,27 @@ struct DirNo {
 template <typename T>
 constexpr int kSumVals = sizeof(T) == 4 ? 32 : 16;
 
-// v[0..NV) of every lane -> lane i holds the sum over lanes of v[i mod NV]: at
-// each step a lane keeps one half of its values and adds the partner's copy of
-// that half (one exchange per value instead of five).
-template <typename T, int NV>
+// Which column a lane keeps at column slot 0: slot k of lane i holds column k ^
+// sum_perm(i), of C columns (2 per map: re, im)
+template <typename T, int C>
+__device__ __forceinline__ int sum_perm(int lane) { return (lane / (kSumVals<T> / C)) & (C - 1); }
+
+// v[k G + i] of every lane, k a column slot and i < G = NV / C -> lane j holds the
+// sum over lanes of value (column j / G, i = j mod G), j < NV.  At each step a
+// lane keeps one half of its values and adds the partner's copy of that half
+// (one exchange per value instead of five).  Which half is a matter of the
+// lane: with the columns in plain order two selects per exchange (62 of the
+// 124 instructions for 32 values, at half the issue rate); in the lane's own
+// order (sum_perm) every lane keeps the lower half of the slots in the steps over
+// columns, 28 of the 31 exchanges at C = 8.  Measured, plain against lane's own order:
+// FP32 analysis of 8 maps at nside 256 180 -> 164 us, of one at nside 1024 1566 ->
+// 1514; FP64, 4 maps at nside 128, L = 511 76 -> 69; spin-1 round trip of 4 fields at
+// nside 128 147 -> 138.
+template <typename T, int NV, int C>
 __device__ __forceinline__ T transpose_sum(T (&v)[NV], int lane) {
 #pragma unroll
     for (int s = NV / 2; s; s >>= 1) {
-        const bool hi = lane & s;
+        const bool hi = s < NV / C && (lane & s);
 #pragma unroll
         for (int i = 0; i < s; ++i) {
             const T keep = hi ? v[i + s] : v[i];
@@ -261,6 +274,7 @@ __global__ void __launch_bounds__(32 * kDirWarps, dir_min_ctas<T, C, R>())
     const double2* nm = norm + mo * Lpad;
     const double2* sm = seeds + (mo * seed_blocks(L) + i0 / kSeedBlock) * NP;
 
+    const int perm = sum_perm<T, C>(lane), acc_lane = (lane % G) * C + lane / G;
     // ring spectra of 32 R pairs: thread = (order j, ring k), 4 orders = 32 (64) contiguous bytes
     auto stage = [&](int pb) {
 #pragma unroll
@@ -326,11 +340,11 @@ __global__ void __launch_bounds__(32 * kDirWarps, dir_min_ctas<T, C, R>())
             const T w = adjoint ? ((m == 0 || m == rings[p].h) ? (T)1 : (T)2) : (T)rings[p].w;
 #pragma unroll
             for (int bb = 0; bb < CB; ++bb) {
-                const cplx<T>* xs = Xs + warp * XS + 32 * r + lane;
-                const cplx<T> a = xs[bb * 32 * R], c = xs[(CB + bb) * 32 * R];
+                const cplx<T>* xs = Xs + warp * XS + 32 * r + lane + (bb ^ (perm >> 1)) * 32 * R;
+                const cplx<T> a = xs[0], c = xs[CB * 32 * R];
                 const cplx<T> sv = cscale(cadd(a, c), w), dv = cscale(csub(a, c), south ? w : (T)0);
-                S[r][bb] = Pair<T>::make(sv.re, sv.im);
-                D[r][bb] = Pair<T>::make(dv.re, dv.im);
+                S[r][bb] = perm & 1 ? Pair<T>::make(sv.im, sv.re) : Pair<T>::make(sv.re, sv.im);
+                D[r][bb] = perm & 1 ? Pair<T>::make(dv.im, dv.re) : Pair<T>::make(dv.re, dv.im);
             }
         }
         __syncthreads();  // every warp has its rings: the next block's spectra land while this one is used
@@ -375,11 +389,11 @@ __global__ void __launch_bounds__(32 * kDirWarps, dir_min_ctas<T, C, R>())
 #pragma unroll
                 for (int bb = 0; bb < CB; ++bb) {
                     const auto q = v[i][bb].get();
-                    f[i * C + 2 * bb] = q.x;
-                    f[i * C + 2 * bb + 1] = q.y;
+                    f[2 * bb * G + i] = q.x;
+                    f[(2 * bb + 1) * G + i] = q.y;
                 }
-            const T sum = transpose_sum(f, lane);  // lane = (degree in group) C + column
-            if (lane < NV) acc[g * NV + lane] += sum;
+            const T sum = transpose_sum<T, NV, C>(f, lane);  // lane = column G + degree in group
+            if (lane < NV) acc[g * NV + acc_lane] += sum;
         };
         const int gs = lmax < 0 ? g : min(ng, (lmax - l0) / G + 1);  // later groups start no ring
 #pragma unroll 1

@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(32 * kDirWarps, vec_min_ctas<T, CV, R>())
     const auto ord = VecGen<T>::order((int)mo, Mv + 1, Lp, Lpad, NP, coef, norm);
     for (int i = lane; i < ng * G; i += 32) fac[i] = VecFac<T>::make(l0 + i, m, nm, Lv);
 
+    const int perm = sum_perm<T, 2 * NC>(lane), acc_lane = (lane % (2 * G)) * 2 * NC + lane / (2 * G);
     auto stage = [&](int pb) {
 #pragma unroll
         for (int kk = 0; kk < R; ++kk) {
@@ -343,11 +344,11 @@ __global__ void __launch_bounds__(32 * kDirWarps, vec_min_ctas<T, CV, R>())
             const T w = (T)(VecGen<T>::kScaled ? w0 * rl.rs : w0);  // quadrature weight (/ sin(theta))
 #pragma unroll
             for (int cc = 0; cc < NC; ++cc) {
-                const cplx<T>* xs = Xs + warp * XS + 32 * r + lane;
-                const cplx<T> a = xs[cc * 32 * R], c = xs[(NC + cc) * 32 * R];
+                const cplx<T>* xs = Xs + warp * XS + 32 * r + lane + (cc ^ (perm >> 1)) * 32 * R;
+                const cplx<T> a = xs[0], c = xs[NC * 32 * R];
                 const cplx<T> sv = cscale(cadd(a, c), w), dv = cscale(csub(a, c), south ? w : (T)0);
-                S[r][cc] = Pair<T>::make(sv.re, sv.im);
-                D[r][cc] = Pair<T>::make(dv.re, dv.im);
+                S[r][cc] = perm & 1 ? Pair<T>::make(sv.im, sv.re) : Pair<T>::make(sv.re, sv.im);
+                D[r][cc] = perm & 1 ? Pair<T>::make(dv.im, dv.re) : Pair<T>::make(dv.re, dv.im);
             }
         }
         __syncthreads();
@@ -388,11 +389,11 @@ __global__ void __launch_bounds__(32 * kDirWarps, vec_min_ctas<T, CV, R>())
 #pragma unroll
                     for (int cc = 0; cc < NC; ++cc) {
                         const auto q = v[i][h][cc].get();
-                        f[(i * 2 + h) * 2 * NC + 2 * cc] = q.x;
-                        f[(i * 2 + h) * 2 * NC + 2 * cc + 1] = q.y;
+                        f[(2 * cc * G + i) * 2 + h] = q.x;
+                        f[((2 * cc + 1) * G + i) * 2 + h] = q.y;
                     }
-            const T sum = transpose_sum(f, lane);
-            if (lane < NV) acc[g * NV + lane] += sum;
+            const T sum = transpose_sum<T, NV, 2 * NC>(f, lane);  // lane = (column G + degree in group) 2 + h
+            if (lane < NV) acc[g * NV + acc_lane] += sum;
         };
         int g = max(0, lmin - l0) / G;
         const int gs = lmax < 0 ? g : min(ng, (lmax - l0) / G + 1);
