@@ -1237,9 +1237,9 @@ struct Pipeline {
     // FP64 synthesis always (nside 256, 32 maps: 957 us against 2583 us of the tiled
     // kernel it replaced) and FP64 analysis up to 48 maps, beyond which the tiled
     // kernel's cost for 64 columns spreads over enough of them (whole calls, direct
-    // against tiled, nside 256: 16 maps 771 / 1748 us, 32 maps 1385 / 1903, 48 maps
-    // 1996 / 2074, 56 maps 2321 / 2175; nside 512: 48 maps 12.7 / 13.1 ms, 64 maps
-    // 16.8 / 13.8); and the FP32 ones in mixed
+    // against tiled, nside 256: 32 maps 1.26 / 1.90 ms, 48 maps 1.82 / 2.07;
+    // nside 512, 48 maps 11.4 / 13.1; and, before sum_perm took 8% off the direct
+    // one, 64 maps 2.6 / 2.3 and 16.8 / 13.8); and the FP32 ones in mixed
     // plans for a few maps, which pay the tensor-core kernels' whole table
     // stream and layout passes (and come out more accurate): whole calls,
     // direct / tensor cores, nside 1024 analysis 2 maps 2.3 / 2.8 ms, 4 maps 3.6 /
@@ -1263,7 +1263,9 @@ struct Pipeline {
     }
     // Degrees per warp of an analysis: long chunks amortise a ring block's set-up,
     // short ones give a small plan more CTAs (`groups` CTAs per chunk; four an SM
-    // wanted).  512 measured slower than 256 (fewer CTAs fit an SM).
+    // wanted).  512 measured slower than 256 (fewer CTAs fit an SM).  Wanting eight
+    // an SM moves single sizes either way (nside 256, FP32: 8 maps 167 -> 173 us, 16
+    // maps 304 -> 277): how the last wave of CTAs falls, not the set-up's share.
     static int degree_chunk(int L, int64_t groups) {
         int lch = kSeedBlock;
         while (2 * lch <= 256 && lch < L && groups * ((L + 2 * lch - 1) / (2 * lch)) >= 4 * 148) lch *= 2;
