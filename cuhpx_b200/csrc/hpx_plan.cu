@@ -1511,13 +1511,20 @@ void set_extents(const hpx_plan_s* P, cudaStream_t st, int64_t map_elems, int64_
 
 // Spin-1 transforms of a plan built with L+1 degrees and M+1 orders (see
 // vector.cuh): maps [batch][2][npix] <-> coefficients [batch][2][L][M].  Each
-// pass takes batch_chunk / 2 vector maps, whose 2 components run through the
-// ring stages as batch_chunk scalar maps.
+// pass takes batch_chunk / 2 vector maps (one at least), whose 2 components run
+// through the ring stages as scalar maps.
+//
+// The ring spectra are all these transforms keep, so they take the workspace from
+// its start.  With batch_chunk = 1 they have to: a vector map is two scalar maps,
+// and the workspace's own region of spectra holds one.  Together with the folded
+// spectra's region (8 NP M values there) it holds both: a map's spectra are 2 Ftot
+// <= 2 (2 NP) (M + 1) values, no more than that region.
 template <typename T>
 int run_vec(hpx_plan_s* P, Op op, const void* in, void* out, int64_t batch, void* ws, cudaStream_t st, int csphase) {
     Pipeline<T> pl(P, ws, st);
     const int Lv = P->L - 1, Mv = P->M - 1;
     const int64_t vc = std::max(1, P->batch_chunk / 2);
+    pl.F = (T*)ws;
     const size_t alm_stride = (size_t)2 * Lv * Mv * 2;
     const size_t map_stride = (size_t)2 * P->npix;
     for (int64_t b0 = 0; b0 < batch; b0 += vc) {
