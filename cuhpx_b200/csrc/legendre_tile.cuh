@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     const int tid = threadIdx.x, NP = geo.NP;
     const int c0 = blockIdx.y * kTileCols, b0 = c0 / 2;  // first column and map
     if ((int)blockIdx.x >= ntiles) {
-        for (int l = blockIdx.x - ntiles; l < L; l += gridDim.x - ntiles)
+        for (int l = blockIdx.x - ntiles; l < min(L, M - 1); l += gridDim.x - ntiles)
             for (int b = b0; b < min(b0 + kTileCols / 2, nmaps); ++b) {
                 cplx<float>* row = (cplx<float>*)alm + ((int64_t)b * L + l) * M;
                 for (int m = l + 1 + tid; m < M; m += blockDim.x)

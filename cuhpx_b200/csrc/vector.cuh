@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(32 * kDirWarps, vec_min_ctas<T, CV, R>())
     const int NP = geo.NP;
     const int b0 = blockIdx.z * CV;
     if ((int)blockIdx.x == nch) {
-        for (int l = blockIdx.y; l < Lv; l += gridDim.y)
+        for (int l = blockIdx.y; l < min(Lv, Mv - 1); l += gridDim.y)
             for (int cc = 0; cc < NC; ++cc) {
                 const int64_t row = (int64_t)(2 * b0 + cc) * Lv + l;
                 if (2 * b0 + cc >= 2 * nvec) break;
