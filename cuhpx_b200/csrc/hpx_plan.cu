@@ -1378,11 +1378,24 @@ struct Pipeline {
                                                            P->d_lstart, P->d_pstart, P->d_alpha, P->d_norm, P->Lpad);
     }
     // The tiled FP32 contractions (legendre_tile.cuh) against the direct ones, whole
-    // calls: analysis nside 256, 32 maps 667 / 694 us, 16 maps 613 / 411; nside
-    // 128, 32 maps 161 / 156, 48 maps 185 / 227; below that the three launches
-    // more decide (nside 64, 48 maps 67 / 66, 64 maps 75 / 77).  Synthesis nside 512, 48
-    // maps 4200 / 4531, 32 maps 3754 / 3044; nside 128, 64 maps 207 / 221.
-    bool tile_fwd(int nb) const { return P->tiled() && nb > (P->NP >= 256 ? 30 : 56); }
+    // calls in us.  Analysis, direct / tiled: nside 512, L = M = 1023 24 maps 2700 /
+    // 3451, 32 maps 3541 / 3586, 40 maps 4389 / 3741; nside 256, L = 511 30 maps 623 /
+    // 649, 40 maps 762 / 697; nside 64, where the three launches more decide until
+    // later, L = 127 48 maps 61 / 63, 64 maps 71 / 68.  Up to 64 degrees half of
+    // every 128-degree block and more would be empty and there are no more blocks than
+    // orders (nside 128, L = 32 48 maps 82 / 100, nside 512, L = 64 64 maps 1005 / 1026);
+    // with one block an order and too few orders for three quarters of the SMs
+    // the same decides while the direct kernel has few rings or maps to repeat its
+    // recurrences for (nside 128, L = 100 64 maps 128 / 132; nside 256, L = 100 64
+    // maps 344 / 334; nside 512, L = 96 48 maps 805 / 823, 64 maps 1082 / 1040).
+    bool tile_fwd(int nb) const {
+        if (!P->tiled() || P->L <= 64 || nb <= (P->NP >= 256 ? 30 : 56)) return false;
+        const int64_t ctas = (int64_t)std::min(P->M, P->L) * ((2 * nb + kTileCols - 1) / kTileCols);
+        return P->L > kTileDeg || ctas > 111 || (P->NP > 256 && nb > 48);
+    }
+    // Synthesis, direct / tiled: nside 512, L = 1023 32 maps 3040 / 3640, 46 maps 4496 /
+    // 3909, L = 256 46 maps 1035 / 1097, 57 maps 1284 / 1276; nside 128, L = 255 48 maps
+    // 172 / 180, 57 maps 207 / 199; nside 64, L = 127 64 maps 66 / 68.
     bool tile_inv(int nb) const { return P->tiled() && P->NP >= 256 && nb > (P->NP >= 512 ? 46 : 56); }
     // alm -> map (ref: residual ref - map)
     void synthesis(const T* alm, T* map, int nb, int adjoint, const T* ref) {
@@ -1430,7 +1443,7 @@ struct Pipeline {
         Timer tm(P, st, kStLegFwd);
         if constexpr (sizeof(T) == 4) {
             const int nj = (P->L + kTileDeg - 1) / kTileDeg, nt = (P->M + 3) / 4 * 4 * nj;
-            k_leg_fwd_tile<<<dim3(nt + (accumulate ? 0 : 148), (C + kTileCols - 1) / kTileCols), kTileThreads,
+            k_leg_fwd_tile<<<dim3(nt + (accumulate ? 0 : 148), (2 * nb + kTileCols - 1) / kTileCols), kTileThreads,
                              kTileFwdSmem, st>>>(spec, C, nb, alm, P->L, P->M, P->geo, P->d_z, P->d_lstart, P->d_pstart,
                                                  P->d_alpha, P->d_norm, P->Lpad, P->d_seeds, nj, nt, accumulate);
         } else {

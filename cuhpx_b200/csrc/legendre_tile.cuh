@@ -20,7 +20,10 @@
 // (the kernel that generated and multiplied in the same threads), synthesis 5694
 // -> 2843 us (that kernel; 5016 us by the direct one), 55% of the FMA rate: what
 // is left is the exposed latency of two multiplying warps a scheduler and
-// the padding of 128-degree blocks.
+// the padding of 128-degree blocks.  Blocks at the end of an order leave out the
+// warps that have no degrees, and the analysis' loaders keep the next stage's rows in
+// flight while they hand one over (whole call of that size 4189 -> 4157 us, nside
+// 256, L = 511 825 -> 806 us; either alone changes nothing).
 #pragma once
 
 #include "legendre_direct.cuh"
@@ -84,10 +87,13 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     const int tid = threadIdx.x, NP = geo.NP;
     const int c0 = blockIdx.y * kTileCols, b0 = c0 / 2;  // first column and map
     if ((int)blockIdx.x >= ntiles) {
+        // a warp per row and map (by whole CTAs, 64 maps one after the other, the rows
+        // took 30 us of 421 at nside 64, L = 127, 512 maps a pass)
+        const int nb = min(kTileCols / 2, nmaps - b0), lane = tid & 31;
         for (int l = blockIdx.x - ntiles; l < min(L, M - 1); l += gridDim.x - ntiles)
-            for (int b = b0; b < min(b0 + kTileCols / 2, nmaps); ++b) {
+            for (int b = b0 + (tid >> 5); b < b0 + nb; b += kTileThreads / 32) {
                 cplx<float>* row = (cplx<float>*)alm + ((int64_t)b * L + l) * M;
-                for (int m = l + 1 + tid; m < M; m += blockDim.x)
+                for (int m = l + 1 + lane; m < M; m += 32)
                     if (HPX_INB(2 * (((int64_t)b * L + l) * M + m) + 1, kExtAlm, 15)) row[m] = {0.f, 0.f};
             }
         return;
@@ -127,9 +133,13 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                     for (int q = 0; q < nr; ++q) cp_async16(Xs + 2 * q * kTileCols, src + (int64_t)q * C);
                 }
                 cp_async_commit();
-                cp_async_wait<0>();
-                tile_arrive(tile_full(st));
+                if (c > 0) {  // hand over the stage before; this one's rows stay in flight
+                    cp_async_wait<1>();
+                    tile_arrive(tile_full((c - 1) % kTileStages));
+                }
             }
+            cp_async_wait<0>();
+            if (nch > 0) tile_arrive(tile_full((nch - 1) % kTileStages));
             return;
         }
         // ---------------------------------------------------- generators: lane = ring, warp = block of 64 degrees
@@ -138,8 +148,14 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         const double* al = alpha + mo + 2 + lb;
         const double2* nm = norm + mo;
         const double2* sp = seeds + ((int64_t)m * seed_blocks(L) + (lb - m) / kSeedBlock) * NP;
-        const bool any = lb < L;
-        const double n0 = any ? nm[lb].y : 0.0, n1 = lb + 1 < L ? nm[lb + 1].y : 0.0;
+        if (lb >= L) {  // no degree of the order, and nobody reads the values
+            for (int c = 0; c < nch; ++c) {
+                if (c >= kTileStages) tile_wait(tile_empty(c % kTileStages));
+                tile_arrive(tile_full(c % kTileStages));
+            }
+            return;
+        }
+        const double n0 = nm[lb].y, n1 = lb + 1 < L ? nm[lb + 1].y : 0.0;
         // a ring's start degree, node and seeds, fetched a stage ahead
         int ls_n = kNoDegree;
         double x_n = 0.0;
@@ -147,7 +163,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         auto fetch = [&](int c) {
             const int p = p0 + c * kTileRing + lane;
             ls_n = kNoDegree;
-            if (any && p < NP) {
+            if (p < NP) {
                 ls_n = lstart[(int64_t)m * NP + p];
                 x_n = z[p];
                 sd_n = sp[p];
@@ -202,6 +218,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     }
     // -------------------------------------------------------- multipliers
     const int par = tid >> 7, tx = tid & 15, ty = (tid >> 4) & 7;
+    const bool rows = l0 + 16 * (ty & ~1) + par < L;  // the warp (two ty) has degrees of the order
     Pair<float> acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -212,7 +229,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         const float* Ps = stages + st * kTileFwdStage + 64 * par + 8 * ty;
         const float* Xs = stages + st * kTileFwdStage + kTileRing * kTilePRow + par * kTileCols + 4 * tx;
         tile_wait(tile_full(st));
-        tile_steps<kTilePRow, 2 * kTileCols>(acc, Ps, Xs, min(kTileRing, NP - p0 - c * kTileRing));
+        if (rows) tile_steps<kTilePRow, 2 * kTileCols>(acc, Ps, Xs, min(kTileRing, NP - p0 - c * kTileRing));
         if (c + kTileStages < nch) tile_arrive(tile_empty(st));
     }
 #pragma unroll
