@@ -1237,25 +1237,41 @@ struct Pipeline {
     // FP64 synthesis always (nside 256, 32 maps: 957 us against 2583 us of the tiled
     // kernel it replaced) and FP64 analysis up to 48 maps, beyond which the tiled
     // kernel's cost for 64 columns spreads over enough of them (whole calls, direct
-    // against tiled, nside 256: 32 maps 1.26 / 1.90 ms, 48 maps 1.82 / 2.07;
-    // nside 512, 48 maps 11.4 / 13.1; and, before sum_perm took 8% off the direct
-    // one, 64 maps 2.6 / 2.3 and 16.8 / 13.8); and the FP32 ones in mixed
-    // plans for a few maps, which pay the tensor-core kernels' whole table
-    // stream and layout passes (and come out more accurate): whole calls,
-    // direct / tensor cores, nside 1024 analysis 2 maps 2.3 / 2.8 ms, 4 maps 3.6 /
-    // 2.9, synthesis 4 maps 2.7 / 3.0, 8 maps 4.8 / 3.3; nside 256 analysis 4 maps
-    // 125 / 135 us, 8 maps 222 / 152, synthesis 8 maps 145 / 163, 12 maps 212 / 183;
-    // nside 64 16 maps 39 / 40 and 33 / 46.  Plans without the table
-    // generate Pbar either way and cross over later.
+    // against tiled: nside 256, L = 511 48 maps 1.81 / 2.06 ms, 56 maps 2.10 / 2.17, 60
+    // maps 2.24 / 2.22; nside 512, L = 1023 48 maps 11.4 / 13.1, 56 maps 13.3 / 13.4, 64
+    // maps 15.1 / 13.8; nside 128, L = 511, M = 257 49 maps 742 / 756 us, 52 maps 767 /
+    // 762); and the FP32 ones in mixed plans for a few maps, which pay the tensor-core
+    // kernels' whole table stream and layout passes (and come out more accurate).
     bool direct_fwd(int nb) const {
-        if (P->mixed()) return nb <= mixed_direct(2, 4, 8);
+        if (P->mixed()) return nb <= mixed_direct(2, 4, 8) && enough_direct_ctas(nb);
         return sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 48;
     }
     bool direct_inv(int nb) const { return P->mixed() ? nb <= mixed_direct(4, 8, 12) : !tile_inv(nb); }
+    // Whole calls, direct / tensor cores with the table: nside 1024, L = 2047 analysis 2
+    // maps 2.1 / 2.8 ms, 4 maps 3.2 / 2.9, synthesis 4 maps 2.6 / 3.0, 8 maps 5.3 / 3.3;
+    // nside 256, L = 511 analysis 4 maps 126 / 131 us, 6 maps 187 / 141, synthesis 8 maps
+    // 141 / 161, 10 maps 209 / 173; nside 64, L = 127 16 maps 35 / 37 and 31 / 41.  Without the
+    // table both generate Pbar, and the direct kernels stay ahead for longer than
+    // these limits ask for: nside 256, L = 511 analysis 8 maps 205 / 305, 12 maps 279 /
+    // 321, synthesis 12 maps 217 / 337, 16 maps 274 / 358; nside 1024, L = 2047 analysis 8
+    // maps 6.2 / 10.1 ms, 12 maps 9.1 / 10.3, synthesis 12 maps 7.7 / 10.1.
     int mixed_direct(int large, int medium, int no_table) const {
         if (kWithholdTmaLoads) return 0;  // the failure-detection build keeps to the pipeline it tests
         if (!P->tc.table) return no_table;
         return P->NP <= 128 ? 16 : P->NP <= 512 ? medium : large;
+    }
+    // A direct analysis walks all rings of its degrees and orders in one CTA: with few
+    // degrees and orders on a large grid it leaves the SMs idle for longer than
+    // the tensor-core kernels' extra passes take (direct / tensor cores with the table,
+    // 16 CTAs: nside 128, L = 64 4 maps 37 / 34 us, nside 256, L = 64 4 maps 69 / 47, nside
+    // 512, L = 64 2 maps 114 / 80, nside 1024, L = 64 2 maps 336 / 211, one map 201 / 163;
+    // without it, nside 512, L = 64 8 maps 250 / 244, nside 1024, L = 64 one map 209 / 285, 4
+    // maps 469 / 428; 256 CTAs, with it: nside 256, L = 256 4 maps 79 / 81).
+    bool enough_direct_ctas(int nb) const {
+        if (P->NP <= (P->tc.table ? 256 : 1024) || (nb == 1 && (!P->tc.table || P->NP <= 512))) return true;
+        const int64_t groups = (int64_t)((P->M + kDirWarps - 1) / kDirWarps) * ((nb + 3) / 4);
+        const int lch = degree_chunk(P->L, groups);
+        return groups * ((P->L + lch - 1) / lch) >= (P->tc.table ? 148 : 48);
     }
     const typename DirRec<T>::Coef* dir_coef() const {
         if constexpr (sizeof(T) == 4) return P->d_alpha;
