@@ -1192,17 +1192,25 @@ __global__ void k_tc_to_alm(const float* __restrict__ ycols, int nmaps, int L, i
     __shared__ float2 tile[NB][33];
     const int m0 = blockIdx.x * 32, l = blockIdx.y;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
-    constexpr int NL = 32 * NB / 256;
+    // W lanes read a row (a warp its two halves one after the other at NB = 64: with the
+    // halves on different warps the pass took 5% longer at nside 256, 64 maps, and
+    // 20% at 17)
+    constexpr int W = NB < 32 ? NB : 32, H = NB / W, RP = 256 / W, K = 32 / RP;
+    const int r = tid / W, c = tid % W;
     // all loads of the thread are issued before the first shared-memory store
-    float2 vv[NL];
+    float2 vv[K][H];
 #pragma unroll
-    for (int k = 0; k < NL; ++k) {
-        const int i = tid + 256 * k, m = m0 + i / NB;
+    for (int k = 0; k < K; ++k) {
+        const int m = m0 + r + RP * k;
         const bool live = m < m_end && m <= l && HPX_INB(((int64_t)m * L + l) * 2 * NB + 2 * NB - 1, kExtYcols, 11);
-        vv[k] = live ? ((const float2*)(ycols + ((int64_t)m * L + l) * 2 * NB))[i % NB] : make_float2(0.f, 0.f);
+        const float2* row = (const float2*)(ycols + ((int64_t)m * L + l) * 2 * NB);
+#pragma unroll
+        for (int h = 0; h < H; ++h) vv[k][h] = live ? row[c + W * h] : make_float2(0.f, 0.f);
     }
 #pragma unroll
-    for (int k = 0; k < NL; ++k) tile[(tid + 256 * k) % NB][(tid + 256 * k) / NB] = vv[k];
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int h = 0; h < H; ++h) tile[c + W * h][r + RP * k] = vv[k][h];
     __syncthreads();
     const int m = m0 + tx;
     if (m >= m_end) return;
