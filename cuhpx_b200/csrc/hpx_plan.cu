@@ -1782,14 +1782,25 @@ struct RemapLaunch {
     RemapSide src, dst;
 };
 
-template <typename E, int SO, int DO>
+template <typename E, int SO, int DO, int R, int MIN_CTAS>
 int launch_remap_async(const E* in, E* out, const RemapLaunch& L) {
-    const int rc = remap_smem_optin<k_remap_async<E, SO, DO>>(L.smem);
+    const int rc = remap_smem_optin<k_remap_async<E, SO, DO, R, MIN_CTAS>>(L.smem);
     if (rc != HPX_OK) return rc;
-    k_remap_async<E, SO, DO><<<L.grid, kRemapThreads, L.smem, L.st>>>(in, out, L.np, L.nside, L.logs, L.log_tiles,
-                                                                      L.nb, L.mpc, L.src, L.dst, L.vec);
+    k_remap_async<E, SO, DO, R, MIN_CTAS><<<L.grid, kRemapThreads, L.smem, L.st>>>(
+        in, out, L.np, L.nside, L.logs, L.log_tiles, L.nb, L.mpc, L.src, L.dst, L.vec);
     HPX_CUDA_TRY(cudaGetLastError());
     return HPX_OK;
+}
+// (pixels a thread and CTAs an SM matter on a RING side only)
+template <typename E, int SO, int DO>
+int launch_remap_async(const E* in, E* out, const RemapLaunch& L) {
+    if constexpr ((SO == kOrderRing || DO == kOrderRing) && sizeof(E) == 4) {
+        if (1 << (2 * L.logs) > kRemapSmall * kRemapThreads) return launch_remap_async<E, SO, DO, kRemapBig, 0>(in, out, L);
+        return launch_remap_async<E, SO, DO, kRemapSmall, kRemapFewCtas>(in, out, L);
+    }
+    if constexpr (DO == kOrderRing && sizeof(E) == 8)
+        if (std::min(L.mpc, L.nb) <= kRemapFewMaps) return launch_remap_async<E, SO, DO, kRemapSmall, kRemapFewCtas>(in, out, L);
+    return launch_remap_async<E, SO, DO, kRemapSmall, 0>(in, out, L);
 }
 
 template <typename E>
@@ -1809,7 +1820,11 @@ int dispatch_remap_async(const E* in, E* out, const RemapLaunch& L) {
 // 32 x 32 above, fewer for nside < 64.  Map groups of up to 16 maps a CTA
 // amortise the offsets' arithmetic, while leaving at least 8 CTAs a
 // multiprocessor (nside 512, 16 float maps, nest2ring / ring2nest: 8 CTAs 104 / 108
-// us, 16 CTAs 112 / 130, 4 CTAs 108 / 107).  Elements of 4, 8 and 16 bytes take the cp.async pipeline
+// us, 16 CTAs 112 / 130, 4 CTAs 108 / 107), 16 of the smaller tiles as long as a CTA
+// keeps two maps (nside 256, 16 maps of 8 bytes, XY to NEST 35 us against 36, of 16 bytes,
+// NEST to RING 70 against 73, but of 8 bytes RING to XY 41 against 39; nside 64, 64 maps of 8 bytes
+// with two a CTA 12.4, one 18.5).
+// Elements of 4, 8 and 16 bytes take the cp.async pipeline
 // (16-byte accesses on NEST and XY sides when the tiles are at least 16 bytes
 // wide and both buffers 16-byte aligned); 1- and 2-byte elements stage
 // through registers.
@@ -1823,6 +1838,8 @@ int launch_remap(const void* in, void* out, int64_t batch, int nside, RemapSide 
     const int64_t tiles = 12ll << (2 * log_tiles);
     int mpc = 16;
     while (mpc > 1 && tiles * ((batch + mpc - 1) / mpc) < 148ll * 8) mpc >>= 1;
+    if (sizeof(E) == 16 || (sizeof(E) == 8 && src.order != kOrderRing))
+        while (mpc > 2 && tiles * ((batch + mpc - 1) / mpc) < 148ll * 16) mpc >>= 1;
     const bool ring = src.order == kOrderRing || dst.order == kOrderRing;
     constexpr bool kAsync = sizeof(E) >= 4;
     const size_t smem = kAsync ? remap_async_smem_bytes(s, (int)sizeof(E), dst.order == kOrderRing)
@@ -1840,15 +1857,16 @@ int launch_remap(const void* in, void* out, int64_t batch, int nside, RemapSide 
             const int rc = dispatch_remap_async<E>(pin, pout, L);
             if (rc != HPX_OK) return rc;
         } else {
+            const bool any = ring || std::min(mpc, nb) > kRemapFewMaps;
             if (s == 64)
-                k_remap<E, 16><<<grid, kRemapThreads, smem, st>>>(pin, pout, np, nside, logs, log_tiles, nb, mpc, src,
-                                                                  dst);
+                (any ? k_remap<E, 16, true> : k_remap<E, 16, false>)<<<grid, kRemapThreads, smem, st>>>(
+                    pin, pout, np, nside, logs, log_tiles, nb, mpc, src, dst);
             else if (s == 32)
-                k_remap<E, 4><<<grid, kRemapThreads, smem, st>>>(pin, pout, np, nside, logs, log_tiles, nb, mpc, src,
-                                                                 dst);
+                (any ? k_remap<E, 4, true> : k_remap<E, 4, false>)<<<grid, kRemapThreads, smem, st>>>(
+                    pin, pout, np, nside, logs, log_tiles, nb, mpc, src, dst);
             else
-                k_remap<E, 1><<<grid, kRemapThreads, smem, st>>>(pin, pout, np, nside, logs, log_tiles, nb, mpc, src,
-                                                                 dst);
+                (any ? k_remap<E, 1, true> : k_remap<E, 1, false>)<<<grid, kRemapThreads, smem, st>>>(
+                    pin, pout, np, nside, logs, log_tiles, nb, mpc, src, dst);
             HPX_CUDA_TRY(cudaGetLastError());
         }
     }

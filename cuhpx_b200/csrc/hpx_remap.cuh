@@ -269,11 +269,16 @@ __device__ __forceinline__ void remap_setup(Tile& t, int nside, int logs, int lo
 // Elements of 1 or 2 bytes: one CTA per (tile, group of maps), R = ceil(s*s /
 // 256) pixels per thread staged through registers; the next map's loads are
 // issued before this map's stores.
-template <typename E, int R>
+// RING = false leaves the RING orders' index arithmetic out, for up to kRemapFewMaps
+// maps a CTA between NEST and XY, where the set-up counts (XY to NEST, nside 8192,
+// one map of bytes 3057 us against 3224); with more maps the compiler's code for
+// the loop over them is the better with it (nside 512, 16 maps 108 against 115).
+template <typename E, int R, bool RING>
 __global__ void __launch_bounds__(kRemapThreads, 5) k_remap(const E* __restrict__ in, E* __restrict__ out,
                                                             int64_t npix, int nside, int logs, int log_tiles,
                                                             int nmaps, int maps_per_cta, RemapSide src,
                                                             RemapSide dst) {
+    __builtin_assume(RING || (src.order != kOrderRing && dst.order != kOrderRing));
     extern __shared__ __align__(16) unsigned char remap_smem[];
     const int s = 1 << logs, ss = s * s;
     E* tile = reinterpret_cast<E*>(remap_smem);
@@ -339,9 +344,16 @@ template <int V>
 HPX_HD int remap_swz(int p) {
     return p ^ (((p >> 5) & (32 / V - 1)) * V);
 }
-// largest tile over the threads: 64 x 64 pixels of 4 bytes, 32 x 32 of 8 and 16
-template <int BYTES>
-constexpr int remap_pixels_per_thread() { return ((BYTES <= 4 ? 64 * 64 : 32 * 32) + kRemapThreads - 1) / kRemapThreads; }
+// Pixels a thread holds on a RING side: 16 for tiles of 64 x 64, up to 4 for smaller
+// ones (the largest of 8- and 16-byte pixels among them).
+constexpr int kRemapBig = 16, kRemapSmall = 4;
+// CTAs an SM that a kernel is compiled for where a CTA's few maps do not outweigh its
+// set-up (0 elsewhere: no bound).  Left alone the compiler takes 60 registers for float64
+// nest2ring and four CTAs fit: 4% to 6% slower for up to 4 maps a CTA (nside 8192, one
+// map 5373 against 5092 us), 8% faster for many (nside 512, 16 maps 182 against 198).
+// Tiles of nside < 64 need it for the same reason: nside 16, 64 float maps 8.2 us on
+// the 64 x 64 instance (80 registers, three CTAs) against 6.2.
+constexpr int kRemapFewMaps = 4, kRemapFewCtas = 6;
 // staged tiles, and the slot table unless a RING destination keeps it in registers
 HPX_HD size_t remap_async_smem_bytes(int s, int elem, bool ring_dst) {
     return kRemapStages * (((size_t)s * s * elem + 15) & ~(size_t)15) + (ring_dst ? 0 : remap_slot_bytes(s));
@@ -364,11 +376,10 @@ __device__ __forceinline__ uint32_t nat_offset(uint32_t base, int p, int logs, i
     return base + (uint32_t)(p >> logs) * (uint32_t)nside + (uint32_t)(p & ((1 << logs) - 1));
 }
 
-template <typename E, int SO, int DO>
-__global__ void __launch_bounds__(kRemapThreads) k_remap_async(const E* __restrict__ in, E* __restrict__ out,
-                                                               int64_t npix, int nside, int logs, int log_tiles,
-                                                               int nmaps, int maps_per_cta, RemapSide src,
-                                                               RemapSide dst, int vec) {
+template <typename E, int SO, int DO, int R, int MIN_CTAS>
+__global__ void __launch_bounds__(kRemapThreads, MIN_CTAS)
+    k_remap_async(const E* __restrict__ in, E* __restrict__ out, int64_t npix, int nside, int logs, int log_tiles,
+                  int nmaps, int maps_per_cta, RemapSide src, RemapSide dst, int vec) {
     static_assert(sizeof(E) == 4 || sizeof(E) == 8 || sizeof(E) == 16, "cp.async moves 4, 8 or 16 bytes");
     static_assert(SO != DO || SO == kOrderXY, "equal orders are a copy");
     constexpr int V = 16 / (int)sizeof(E);
@@ -378,7 +389,6 @@ __global__ void __launch_bounds__(kRemapThreads) k_remap_async(const E* __restri
     uint16_t* sslot = reinterpret_cast<uint16_t*>(remap_smem + kRemapStages * tb);
     // a thread's pixels on a RING side: offsets (and, for a RING destination, the
     // staged slots they read) stay in registers for all maps of the CTA
-    constexpr int R = remap_pixels_per_thread<sizeof(E)>();
     uint32_t roff[R], rslot[R];
     // RING side: the tables are formed (by a rolled loop: the index arithmetic
     // unrolled over a thread's pixels cost more in instruction fetches than the
