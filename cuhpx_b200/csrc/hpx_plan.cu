@@ -1389,7 +1389,9 @@ struct Pipeline {
                                                                                      P->Lpad, (float*)almT, C);
         }
         Timer tm(P, st, kStLegInv);
-        k_leg_inv_tile<<<dim3((P->NP + kTileInvRing - 1) / kTileInvRing, P->M, (2 * nb + kTileCols - 1) / kTileCols),
+        // orders that some ring carries (the others' sums are read by nobody, and 65536
+        // orders are more than a grid's y takes)
+        k_leg_inv_tile<<<dim3((P->NP + kTileInvRing - 1) / kTileInvRing, P->mtmax, (2 * nb + kTileCols - 1) / kTileCols),
                          kTileThreads, kTileInvSmem, st>>>((const float*)almT, C, (float*)spec, P->L, P->M, P->geo, P->d_z,
                                                            P->d_lstart, P->d_pstart, P->d_alpha, P->d_norm, P->Lpad);
     }
