@@ -1526,6 +1526,7 @@ void set_extents(const hpx_plan_s* P, cudaStream_t st, int64_t map_elems, int64_
     v[kExtYcols] = (long long)(P->ycols_bytes() / sizeof(float));
     v[kExtOperA] = P->mixed() ? (long long)2 * P->M * P->tc.Lh * kTcCols : 0;
     v[kExtOperX] = P->mixed() ? (long long)2 * P->M * P->NP * kTcCols / 2 : 0;
+    v[kExtAlmT] = P->tiled() ? (long long)(P->almT_bytes() / sizeof(float)) : 0;
     if (const char* e = getenv("HPX_TEST_SHRINK_EXTENT")) {
         const int k = atoi(e);
         if (k >= 0 && k < kExtN && v[k] > 0) v[k] -= 1;

@@ -130,7 +130,9 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                 const float* src = spec + (((int64_t)m * 2 + par) * NP + pc) * C + c0 + 4 * lane;
                 if (c0 + 4 * lane < C) {  // (columns past C are never written out)
 #pragma unroll 8
-                    for (int q = 0; q < nr; ++q) cp_async16(Xs + 2 * q * kTileCols, src + (int64_t)q * C);
+                    for (int q = 0; q < nr; ++q)
+                        if (HPX_INB(src + (int64_t)q * C + 3 - spec, kExtSpec, 29))
+                            cp_async16(Xs + 2 * q * kTileCols, src + (int64_t)q * C);
                 }
                 cp_async_commit();
                 if (c > 0) {  // hand over the stage before; this one's rows stay in flight
@@ -283,7 +285,8 @@ __global__ void __launch_bounds__(256) k_alm_to_tile(const float* __restrict__ a
         const int i = (tid >> 5) + 8 * k, mm = m0 + i;
         if (mm > l || mm >= M || 2 * b0 + 4 * tx >= C) continue;
         const cplx<float> a = tile[2 * tx][i], b = tile[2 * tx + 1][i];
-        *(float4*)(almT + ((int64_t)mm * L + l) * C + 2 * b0 + 4 * tx) = make_float4(a.re, a.im, b.re, b.im);
+        const int64_t o = ((int64_t)mm * L + l) * C + 2 * b0 + 4 * tx;
+        if (HPX_INB(o + 3, kExtAlmT, 31)) *(float4*)(almT + o) = make_float4(a.re, a.im, b.re, b.im);
     }
 }
 
@@ -320,7 +323,9 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                 const float* src = almT + ((int64_t)m * L + lc) * C + c0 + 4 * lane;
                 if (c0 + 4 * lane < C) {
 #pragma unroll 8
-                    for (int i = w; i < nl; i += 2) cp_async16(As + i * kTileCols, src + (int64_t)i * C);
+                    for (int i = w; i < nl; i += 2)
+                        if (HPX_INB(src + (int64_t)i * C + 3 - almT, kExtAlmT, 30))
+                            cp_async16(As + i * kTileCols, src + (int64_t)i * C);
                 }
                 cp_async_commit();
                 cp_async_wait<0>();
