@@ -320,17 +320,18 @@ def run_gpu(args):
     stats = plan.stats_read()
     plan.stats_enable(False)
     plan.check()  # raises if a tensor-core pipeline wait gave up during the timed steps
-    # the timed result must be a real transform: compare one batch with the plain FP32 path
+    # the timed result must be a real transform: the timed batch (fewer maps would take other
+    # kernels), its first maps compared with the plain FP32 path
     with torch.no_grad():
         ref = hpx.SHTCUDA(nside, lmax=L, mmax=L, precision="fp32")(f[:4])
-        got = sht(f[:4])
+        got = sht(f)[:4]
         plan.check()
         check_rel = float((got - ref).abs().pow(2).sum().sqrt() / ref.abs().pow(2).sum().sqrt())
     if not (check_rel < 1e-3):
         raise RuntimeError(f"timed transform disagrees with the FP32 path: rel-L2 {check_rel:.3e}")
     ms_step = ms / args.steps
     value = world * B * args.steps / (ms / 1000.0)
-    launches_per_step = sum(v[0] * kernels_in_stage(k, prec, nside) for k, v in stats.items()) / args.steps
+    launches_per_step = sum(v[0] * kernels_in_stage(k, prec, nside, B) for k, v in stats.items()) / args.steps
 
     # roofline of the dominant kernel
     roof = roofline(stats, args, prec, refine, nside, L, B, plan.table_bytes > 0, plan.table_stream_bytes)
@@ -372,7 +373,7 @@ def run_gpu(args):
 
     acc = None
     if not args.no_accuracy:
-        acc = accuracy_vs_fp64(torch, hpx, sht, isht, f[: args.accuracy_maps], nside, L, refine, args.spot_maps)
+        acc = accuracy_vs_fp64(torch, hpx, sht, isht, f, args.accuracy_maps, nside, L, refine, args.spot_maps)
 
     # the workload's refined variants: k Jacobi iterations in the analysis (each
     # one more synthesis and analysis of the residual), the same maps, and their
@@ -390,7 +391,7 @@ def run_gpu(args):
             ms_k = time_steps(torch, step_k, max(2, args.steps // 2), args.warmup, dist, stream)
             e = {"maps_per_s": B * max(2, args.steps // 2) / (ms_k / 1000.0)}
             if not args.no_accuracy:
-                a_k = accuracy_vs_fp64(torch, hpx, sht_k, isht, f[: args.accuracy_maps], nside, L, k)
+                a_k = accuracy_vs_fp64(torch, hpx, sht_k, isht, f, args.accuracy_maps, nside, L, k)
                 e["roundtrip_rel_l2"] = a_k["roundtrip_rel_l2"]
                 e["alm_rel_l2"] = a_k["alm_rel_l2"]
             refined[str(k)] = e
@@ -456,10 +457,10 @@ def run_gpu(args):
     return 0
 
 
-def accuracy_vs_fp64(torch, hpx, sht, isht, f, nside, L, refine, spot_maps=0):
+def accuracy_vs_fp64(torch, hpx, sht, isht, f, maps, nside, L, refine, spot_maps=0):
     """Rel-L2 of the timed modules against the FP64 path with the same Jacobi
-    iterations, on the first maps of the timed batch: the analysis coefficients
-    and the round trip iSHT(SHT(f)).  With spot_maps > 0 (no refinement), the
+    iterations: the analysis coefficients and the round trip iSHT(SHT(f)) of the
+    timed batch f (a smaller one would take other kernels), its first maps compared.  With spot_maps > 0 (no refinement), the
     orders 0, 1, 2, M/4, M/2 and M-1 of the first spot_maps maps are also
     compared with the CPU spot oracle (one float64 Legendre column at a time,
     oracle/hpx_oracle.py sht_spot), for the timed path and the FP64 path."""
@@ -468,13 +469,15 @@ def accuracy_vs_fp64(torch, hpx, sht, isht, f, nside, L, refine, spot_maps=0):
         return float((a.to(b.dtype) - b).abs().pow(2).sum().sqrt() / b.abs().pow(2).sum().sqrt())
 
     with torch.no_grad():
-        f64 = f.double()
+        f64 = f[:maps].double()
         a64 = hpx.SHTCUDA(nside, lmax=L, mmax=L, refine_iters=refine)(f64)
         r64 = hpx.iSHTCUDA(nside, lmax=L, mmax=L)(a64)
         a = sht(f)
-        r = isht(a)
+        r = isht(a)[:maps]
+        a = a[:maps]
         out = {
-            "maps": int(f.shape[0]),
+            "maps": int(f64.shape[0]),
+            "batch": int(f.shape[0]),
             "refine_iters": refine,
             "alm_rel_l2": rel(a, a64),
             "roundtrip_rel_l2": rel(r, r64),
@@ -642,12 +645,28 @@ def ring_kernel_count(nside):
     return len(kinds)
 
 
-# kernels behind each stage's timer: the ring stages launch one kernel per ring
-# list, and the mixed path's alm_to_columns is a max scan plus the conversion
-# when the operand carries a per-map fp16 scale
-def kernels_in_stage(name, prec, nside):
+def ring_launches(nside, maps):
+    """Ring kernels a pass of `maps` maps launches: one per ring list, or a single one
+    for the two common lists of a small pass (k_ring_*_any: up to 16 maps and 1200
+    CTAs of both rings of a pair and at most 8 maps, halved while they leave less
+    than one CTA on each of 148 SMs)."""
+    lists = ring_kernel_count(nside)
+    if maps > 16 or lists != 2:  # (with the 3072-point list there are three)
+        return lists
+    pairs, per = 2 * nside, 8
+    while per > 1 and pairs * -(-maps // per) < 148:
+        per //= 2
+    return 1 if pairs * -(-maps // per) <= 1200 else lists
+
+
+# kernels behind each stage's timer (mean over a batch's passes of 64 maps): the ring
+# stages launch one kernel per ring list or one for a small pass, and the mixed path's
+# alm_to_columns is a max scan plus the conversion when the operand carries a
+# per-map fp16 scale
+def kernels_in_stage(name, prec, nside, batch=64):
     if name.startswith("ring_fft"):
-        return ring_kernel_count(nside)
+        passes = [64] * (batch // 64) + ([batch % 64] if batch % 64 else [])
+        return sum(ring_launches(nside, n) for n in passes) / len(passes)
     return 2 if (name == "alm_to_columns" and prec == "f16x3") else 1
 
 
