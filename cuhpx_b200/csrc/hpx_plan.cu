@@ -117,7 +117,7 @@ struct hpx_plan_s {
     int Lpad = 0;                // coefficient row length (L + kCoefPad)
     double2* d_coef = nullptr;   // [M][Lpad] recurrence coefficients
     double2* d_seeds = nullptr;  // [M][seed_blocks(L)][2*nside] block seeds
-    int2* d_fwdtiles = nullptr;  // (m, degree block) tiles of the forward contraction
+    int2* d_fwdtiles = nullptr;  // (m, degree block) tiles of the FP64 analysis of many maps
     double* d_z = nullptr;       // cos(theta) of the north rings
     RingLite* d_lite = nullptr;  // ring pairs as the direct contractions read them
     double* d_alpha = nullptr;   // [M][Lpad] FP32 recurrence coefficients (legendre_direct.cuh)
@@ -241,7 +241,8 @@ std::vector<const void*> ring_kernels() {
             (const void*)k_ring_inv<T, 1, false>,  (const void*)k_ring_inv<T, 2, false>};
 }
 
-// largest L the plans accept
+// largest L the plans accept (their long-standing limit; no contraction's shared memory
+// grows with L)
 template <typename T>
 constexpr int max_degrees() { return sizeof(T) == 4 ? 12956 : 11420; }
 
@@ -336,9 +337,12 @@ int create_typed(hpx_plan_s* P) {
     if (P->f64) P->fwd_smem = fwd_smem_bytes<T>();
     int dev_max = 0;
     HPX_CUDA_TRY(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device));
+    if (P->L > max_degrees<T>())
+        return set_err(HPX_ERR_UNSUPPORTED,
+                       "lmax too large: plans of this precision take up to " + std::to_string(max_degrees<T>()) + " degrees");
     if ((int)P->ring_smem > dev_max || (int)P->blue_smem > dev_max || (int)P->blue3_smem > dev_max ||
-        (int)P->fwd_smem > dev_max || P->L > max_degrees<T>())
-        return set_err(HPX_ERR_UNSUPPORTED, "nside/lmax too large for the shared-memory kernels of this precision");
+        (int)P->fwd_smem > dev_max)
+        return set_err(HPX_ERR_UNSUPPORTED, "nside too large for the shared-memory ring kernels of this precision");
     // The attribute is per function, not per plan: always raise it to the device
     // maximum so that a plan needing less never lowers it under another plan.
     HPX_CUDA_TRY(cudaStreamCreateWithFlags(&P->aux, cudaStreamNonBlocking));
@@ -976,7 +980,7 @@ int plan_build(hpx_plan_s* P) {
     e2 = cudaDeviceSynchronize();
     if (e != cudaSuccess || e2 != cudaSuccess)
         return set_err(HPX_ERR_CUDA, std::string("legendre seeds: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
-    {
+    if (P->f64) {
         std::vector<int2> tiles;
         for (int m = 0; m < P->M; ++m) {
             const int nb = m < P->L ? (P->L - m + kSeedBlock - 1) / kSeedBlock : 1;

@@ -184,7 +184,7 @@ __global__ void k_legendre_alpha(int M, int L, int Lpad, const double2* __restri
     }
 }
 
-// ------------------------------------------------------------ forward (analysis)
+// ------------------------------------------------------------ FP64 analysis of many maps
 // alm[b][l][m] = sum_{p >= t0(m)} Pbar_l^m(x_p) X[m][(l-m)&1][p][2b..2b+1]
 // One CTA per (m, degree block of 64, column tile of 128 = 64 maps).  Each
 // pass generates Pbar for RB rings x 64 degrees from the FP64 block seeds
@@ -194,7 +194,7 @@ template <typename T>
 struct FwdCfg {
     static constexpr int LT = kSeedBlock;               // degrees per tile (32 even, 32 odd)
     static constexpr int CT = 128;                      // columns per CTA
-    static constexpr int RB = sizeof(T) == 4 ? 256 : 128;  // rings generated per pass
+    static constexpr int RB = 128;                      // rings generated per pass
     static constexpr int KC = 16;                       // rings per staged X chunk
     static constexpr int LTP = LT + 16 / sizeof(T);     // padded P row
 };
@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(256) k_leg_fwd_simt(const T* __restrict__ spec
     if (!accumulate && jb == 0) {
         for (int i = tid; i < min(m, L) * (CT / 2); i += blockDim.x) {
             const int l = i / (CT / 2), b = c0 / 2 + i % (CT / 2);
-            if (b < nmaps) *(cplx<T>*)(alm + 2 * (((int64_t)b * L + l) * M + m)) = {(T)0, (T)0};
+            const int64_t o = 2 * (((int64_t)b * L + l) * M + m);
+            if (b < nmaps && HPX_INB(o + 1, kExtAlm, 32)) *(cplx<T>*)(alm + o) = {(T)0, (T)0};
         }
     }
     if (m >= L) return;

@@ -109,7 +109,7 @@ struct __align__(16) RingLite {
 //   double: Pbar_l = a_l x Pbar_{l-1} - b_l Pbar_{l-2} as everywhere else;
 //   float:  Pbar_l = c_l q_l with c_l = b_l c_{l-2}, c_m = c_{m+1} = 1, so that
 //           q_l = alpha_l x q_{l-1} - q_{l-2}: two FP64 operations per value
-//           instead of three.  c_l (between about 0.05 and 1) is applied in FP64 once
+//           instead of three.  c_l (between about 0.1 and 1.13) is applied in FP64 once
 //           per degree: to the finished sums (analysis) or to the coefficients
 //           (synthesis).  Past l = L - 1 alpha is zero and q only alternates in sign.
 template <typename T>

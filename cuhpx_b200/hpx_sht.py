@@ -17,11 +17,15 @@ Differences from the reference, all deliberate:
 
 * transforms run on the *current* CUDA stream at call time (the reference
   pins the stream that was current at construction);
+* a map's result depends, within the precision's rounding, on how many maps it is
+  transformed with: the kernels are chosen by that number (equal calls give equal
+  bits);
 * gradients are the exact adjoints of the transforms (the reference's
   hand-written backward is approximate, cuhpx/hpx_sht.py:565-583, 614-641);
 * keyword-only extras: ``precision`` ('fp32'; 'f16x3' or 'bf16x3': tcgen05
   tensor cores with a three-term fp16 (per-map power-of-two scaled, ~22-bit)
-  or bf16 (~16-bit) split and FP32 accumulation),
+  or bf16 (~16-bit) split and FP32 accumulation; a few maps at a time take the
+  FP32 contraction, faster and more accurate there),
   ``refine_iters`` (Jacobi refinement of the analysis), ``batch_chunk``,
   ``legendre_table`` (tensor-core plans: keep the Legendre values resident on
   the device when they fit, default; False generates them on the fly),
@@ -46,7 +50,7 @@ _plans = {}
 class Plan:
     """One ``hpx_plan_t``: immutable, shareable between modules and streams."""
 
-    _ws_last = (None, 0)  # (batch, workspace bytes) of the last call
+    _ws_bytes = None  # workspace bytes, the same for every batch (it is processed in passes)
 
     def __init__(self, nside, lmax, mmax, quad_weights="ring", precision="fp32", device=0, batch_chunk=64, refine_iters=0,
                  legendre_table=True):
@@ -120,12 +124,11 @@ class Plan:
 
     # ------------------------------------------------------------------ calls
     def workspace_bytes(self, batch):
-        last = self._ws_last
-        if last[0] != batch:  # the plan is immutable: so is its answer for a batch
+        if self._ws_bytes is None:  # the plan is immutable: so is its answer
             n = ctypes.c_size_t()
             _lib.check(self._lib.hpx_workspace_size(self._h, int(batch), ctypes.byref(n)), self._h)
-            self._ws_last = last = (batch, n.value)
-        return last[1]
+            self._ws_bytes = n.value
+        return self._ws_bytes
 
     def _call(self, fn, src, dst, batch, *extra):
         # At small sizes the call is bound by the host: plain integers for pointers

@@ -53,9 +53,16 @@ typedef enum {
 } hpx_status_t;
 
 /* Arithmetic of the Legendre contraction.  FFT stages run in float for
- * FP32/BF16X3/F16X3/TF32 plans and in double for FP64 plans. */
+ * FP32/BF16X3/F16X3/TF32 plans and in double for FP64 plans.
+ *
+ * The kernels are chosen by the plan's sizes and by how many maps a pass (up to
+ * batch_chunk maps) holds.  A map's result is therefore the same, bit for bit, in
+ * equal calls and in passes of as many maps, but within the precision's rounding
+ * only where it comes in a pass of another number.  BF16X3 and F16X3 plans
+ * transform passes of a few maps (at most 16; fewer on larger grids) with the FP32
+ * contraction, which is the faster and the more accurate one there. */
 typedef enum {
-    HPX_PREC_FP32 = 0,   /* FP32 SIMT contraction ("plain FP32 path") */
+    HPX_PREC_FP32 = 0,   /* FP32 contraction on CUDA cores ("plain FP32 path") */
     HPX_PREC_FP64 = 1,   /* FP64 everywhere (double I/O)              */
     HPX_PREC_BF16X3 = 2, /* tcgen05 BF16 3-term split (hi*hi + hi*lo + lo*hi),
                             FP32 accumulate; ~16-bit operands          */
