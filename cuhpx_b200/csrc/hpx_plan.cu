@@ -1247,7 +1247,7 @@ struct Pipeline {
     // 762); and the FP32 ones in mixed plans for a few maps, which pay the tensor-core
     // kernels' whole table stream and layout passes (and come out more accurate).
     bool direct_fwd(int nb) const {
-        if (P->mixed()) return nb <= mixed_direct(2, 4, 8) && enough_direct_ctas(nb);
+        if (P->mixed()) return nb <= mixed_direct(2, 4, 8);
         return sizeof(T) == 4 ? !tile_fwd(nb) : nb <= 48;
     }
     bool direct_inv(int nb) const { return P->mixed() ? nb <= mixed_direct(4, 8, 12) : !tile_inv(nb); }
@@ -1263,19 +1263,6 @@ struct Pipeline {
         if (kWithholdTmaLoads) return 0;  // the failure-detection build keeps to the pipeline it tests
         if (!P->tc.table) return no_table;
         return P->NP <= 128 ? 16 : P->NP <= 512 ? medium : large;
-    }
-    // A direct analysis walks all rings of its degrees and orders in one CTA: with few
-    // degrees and orders on a large grid it leaves the SMs idle for longer than
-    // the tensor-core kernels' extra passes take (direct / tensor cores with the table,
-    // 16 CTAs: nside 128, L = 64 4 maps 37 / 34 us, nside 256, L = 64 4 maps 69 / 47, nside
-    // 512, L = 64 2 maps 114 / 80, nside 1024, L = 64 2 maps 336 / 211, one map 201 / 163;
-    // without it, nside 512, L = 64 8 maps 250 / 244, nside 1024, L = 64 one map 209 / 285, 4
-    // maps 469 / 428; 256 CTAs, with it: nside 256, L = 256 4 maps 79 / 81).
-    bool enough_direct_ctas(int nb) const {
-        if (P->NP <= (P->tc.table ? 256 : 1024) || (nb == 1 && (!P->tc.table || P->NP <= 512))) return true;
-        const int64_t groups = (int64_t)((P->M + kDirWarps - 1) / kDirWarps) * ((nb + 3) / 4);
-        const int lch = degree_chunk(P->L, groups);
-        return groups * ((P->L + lch - 1) / lch) >= (P->tc.table ? 148 : 48);
     }
     const typename DirRec<T>::Coef* dir_coef() const {
         if constexpr (sizeof(T) == 4) return P->d_alpha;
@@ -1316,12 +1303,23 @@ struct Pipeline {
     // and where R = 4 leaves a small plan too few warps: analysis with one block
     // of 64 ring pairs (nside 32: 10.6 us against 12.4), synthesis below three
     // CTAs an SM (nside 128, 8 maps: 30 us against 36).
+    // A CTA walks all rings of its degrees and orders, so with few of both most SMs
+    // idle; there the maps are shared among more CTAs, two or one each, until there is
+    // a CTA an SM (whole calls, with / without: nside 1024, L = 64 2 maps 281 / 336 us, 4
+    // maps 366 / 462; nside 256, L = 64 4 maps 49 / 69; nside 128, L = 64 16 maps 49 / 52;
+    // FP64 nside 256, L = 64 4 maps 72 / 85).
     void leg_fwd_direct(T* alm, int nb, int adjoint, int accumulate) {
         Timer tm(P, st, kStLegFwd);
         const bool small = P->NP <= 64;
-        if (nb == 1) {
+        auto idle = [&](int maps) {  // with `maps` maps a CTA
+            const int64_t groups = (int64_t)((P->M + kDirWarps - 1) / kDirWarps) * ((nb + maps - 1) / maps);
+            const int lch = degree_chunk(P->L, groups);
+            return groups * ((P->L + lch - 1) / lch) < 148;
+        };
+        const bool two = nb == 2 || sizeof(T) == 8 || idle(4);
+        if (nb == 1 || (two && idle(2))) {
             small ? leg_fwd_direct_launch<2, 2>(alm, nb, adjoint, accumulate) : leg_fwd_direct_launch<2, 4>(alm, nb, adjoint, accumulate);
-        } else if (nb == 2 || sizeof(T) == 8) {
+        } else if (two) {
             // FP64: two maps at a time leave room for R = 4 (nside 512, 4 maps:
             // 1069 us against 1490 with four maps and R = 2; nside 128, degrees < 511,
             // 4 maps: 76 against 88)
