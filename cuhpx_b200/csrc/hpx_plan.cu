@@ -1357,7 +1357,9 @@ struct Pipeline {
     }
     // Two vector maps at a time (8 columns of each kind) and R as for the scalar
     // contractions (nside 256, 16 maps, FP32: analysis 1208 us with R = 4, 1719
-    // with 2; nside 128, 4 maps, synthesis 60 against 48 us: too few CTAs with 4).
+    // with 2; nside 128, 4 maps, synthesis 60 against 48 us: too few CTAs with 4).  FP64:
+    // R = 2, as R = 4 spills (whole calls, R = 2 / 4: nside 256, 16 maps analysis 4517 / 7829 us,
+    // synthesis 1795 / 4668), but the analysis of one map (361 / 356).
     void vleg_fwd(T* alm, int nb, int csphase, int adjoint, int use_nf) {
         Timer tm(P, st, kStLegFwd);
         constexpr int R2 = sizeof(T) == 4 ? 4 : 2;
